@@ -611,6 +611,17 @@ int repack(lynx_ctx* c, Dst* dst, int dnxp, long long dld, const Src* src, int s
     return LYNX_OK;
 }
 
+// Uploads a host table into a buffer of its own, complete on return.  On the context's stream and
+// waited for: a plain cudaMemcpy from pageable memory may return while its copy is still under way
+// on the legacy stream, which kernels on a non-blocking stream do not wait for.
+int upload_table(lynx_ctx* c, DevBuf& b, const void* src, size_t bytes) {
+    LYNX_TRY(b.ensure(std::max<size_t>(bytes, 16)));
+    if (!bytes) return LYNX_OK;
+    LYNX_CUDA_TRY(cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, c->stream));
+    LYNX_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    return LYNX_OK;
+}
+
 // Nonlocal tables whose grid indices address rows of length nxp.
 int nl_for(lynx_ctx* c, int nxp, const NLDev** out) {
     if (nxp == c->nx) {
@@ -635,13 +646,11 @@ int nl_for(lynx_ctx* c, int nxp, const NLDev** out) {
     const std::vector<int> gp = remap(c->h_gpos), pg = remap(c->h_pt_grid);
     c->nl_layout_bufs.emplace_back();
     DevBuf& b1 = c->nl_layout_bufs.back();
-    LYNX_TRY(b1.ensure(std::max<size_t>(gp.size() * 4, 16)));
-    LYNX_CUDA_TRY(cudaMemcpy(b1.p, gp.data(), gp.size() * 4, cudaMemcpyHostToDevice));
+    LYNX_TRY(upload_table(c, b1, gp.data(), gp.size() * 4));
     d.gpos = b1.as<int>();
     c->nl_layout_bufs.emplace_back();
     DevBuf& b2 = c->nl_layout_bufs.back();
-    LYNX_TRY(b2.ensure(std::max<size_t>(pg.size() * 4, 16)));
-    LYNX_CUDA_TRY(cudaMemcpy(b2.p, pg.data(), pg.size() * 4, cudaMemcpyHostToDevice));
+    LYNX_TRY(upload_table(c, b2, pg.data(), pg.size() * 4));
     d.pt_grid = b2.as<int>();
     c->nl_layouts[nxp] = d;
     *out = &c->nl_layouts[nxp];
@@ -670,11 +679,8 @@ int nl_map_for(lynx_ctx* c, int nxp, const lynx_ctx::NLMap** out) {
         m.rowstart_h[row + 1]++;
     }
     for (long long r = 0; r < rows; ++r) m.rowstart_h[r + 1] += m.rowstart_h[r];
-    LYNX_TRY(m.ptmap.ensure(pm.size() * sizeof(int)));
-    LYNX_CUDA_TRY(cudaMemcpy(m.ptmap.p, pm.data(), pm.size() * sizeof(int), cudaMemcpyHostToDevice));
-    LYNX_TRY(m.rowstart.ensure(m.rowstart_h.size() * sizeof(int)));
-    LYNX_CUDA_TRY(cudaMemcpy(m.rowstart.p, m.rowstart_h.data(), m.rowstart_h.size() * sizeof(int),
-                             cudaMemcpyHostToDevice));
+    LYNX_TRY(upload_table(c, m.ptmap, pm.data(), pm.size() * sizeof(int)));
+    LYNX_TRY(upload_table(c, m.rowstart, m.rowstart_h.data(), m.rowstart_h.size() * sizeof(int)));
     *out = &m;
     return LYNX_OK;
 }
@@ -1828,8 +1834,7 @@ int lynx_set_nonlocal(lynx_ctx* c, int n_img, const int* img_atom, const int* im
     auto up = [&](const void* src, size_t bytes, void** dst) -> int {
         c->nl_bufs.emplace_back();
         DevBuf& b = c->nl_bufs.back();
-        LYNX_TRY(b.ensure(std::max<size_t>(bytes, 16)));
-        if (bytes) LYNX_CUDA_TRY(cudaMemcpy(b.p, src, bytes, cudaMemcpyHostToDevice));
+        LYNX_TRY(upload_table(c, b, src, bytes));
         *dst = b.p;
         return LYNX_OK;
     };
