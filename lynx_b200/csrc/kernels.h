@@ -6,6 +6,8 @@
 
 namespace lynxb {
 
+template <typename T> struct ScalarOf;
+
 constexpr int kMaxR1 = 9;  // FD half-width bound + 1 (coefficient arrays 0..R)
 
 // Geometry + FD coefficients of one cell for the fused stencil kernel.
@@ -235,6 +237,15 @@ constexpr int kExpTilePts = 512;
 template <typename T>
 int launch_nl_gather(const NLDev& nl, const T* x, long long ld, int ncol, T* alpha, int ncolp, double dV,
                      cudaStream_t st);
+// Few atoms: a gather by (atom, 64 columns) leaves most SMs idle, and one kernel can take an atom's
+// gather and its term together.
+constexpr int kNLFewAtoms = 32;
+bool nl_few_atoms(const NLDev& nl);
+// out += scale * chi Gamma dV chi^T x in one kernel (disjoint spheres: nl.compact, at most 32
+// projectors per atom); bitwise launch_nl_gather + launch_nl_scatter for few atoms and complex data.
+template <typename T>
+int launch_nl_apply(const NLDev& nl, const T* x, long long ld, T* out, long long ldo, int ncol, double dV,
+                    typename ScalarOf<T>::type scale, cudaStream_t st);
 template <typename T, typename S>
 int launch_nl_scatter(const NLDev& nl, T* out, long long ld, int ncol, const T* alpha, int ncolp, S scale,
                       cudaStream_t st);

@@ -816,13 +816,15 @@ int cheb_step(lynx_ctx* c, int nxp, const T* x, long long ldx, const T* xold, lo
     // Fused nonlocal term: real data, periodic cell, pipelined kernel, disjoint spheres.  The
     // values (chi alpha) are expanded to the compact point numbering and added by the stencil
     // kernel itself (out += a * W), in the order the separate scatter would add them.
-    const bool fuse = c->has_nl && c->fuse_nl && c->orth && pipe_ok && !ScalarOf<T>::cplx && !use_k && c->nl.compact &&
+    // Few atoms: one kernel after the stencil does the gather and the term together.
+    const bool few = c->has_nl && c->nl.compact && c->nl.max_np <= 32 && nl_few_atoms(c->nl);
+    const bool fuse = c->has_nl && !few && c->fuse_nl && c->orth && pipe_ok && !ScalarOf<T>::cplx && !use_k && c->nl.compact &&
                       c->nl.n_colors == 1 && geom(c).R == 6 && c->bc[0] == LYNX_BC_PERIODIC &&
                       c->bc[1] == LYNX_BC_PERIODIC && c->bc[2] == LYNX_BC_PERIODIC;
     const long long ldw = ((long long)c->nl.n_pts + 3) & ~3LL;  // compact column stride
     const NLDev* nl = nullptr;
-    if (c->has_nl) {
-        LYNX_TRY(nl_for(c, nxp, &nl));
+    if (c->has_nl) LYNX_TRY(nl_for(c, nxp, &nl));
+    if (c->has_nl && !few) {
         LYNX_TRY(c->alpha.ensure(sizeof(T) * (size_t)c->nl.total_proj * ncolp));
         if (fuse && xs_in) {
             // gather from the dense compact copy: entries index it through ent_pt
@@ -866,7 +868,8 @@ int cheb_step(lynx_ctx* c, int nxp, const T* x, long long ldx, const T* xold, lo
         LYNX_TRY(launch_nonorth_terms<T>(ng, nxp, x, ldx, c->gradbuf[0].as<T>(), c->gradbuf[1].as<T>(), ldg, out, ldout,
                                          ncol, a, phl, phr, c->stream));
     }
-    if (c->has_nl)
+    if (few) LYNX_TRY(launch_nl_apply<T>(*nl, x, ldx, out, ldout, ncol, c->dV, (S)a, c->stream));
+    else if (c->has_nl)
         LYNX_TRY(launch_nl_scatter<T, S>(*nl, out, ldout, ncol, c->alpha.as<T>(), ncolp, (S)a, c->stream));
     return LYNX_OK;
 }
@@ -880,7 +883,7 @@ template <typename T>
 int compact_bufs(lynx_ctx* c, int ncol, T* xs[2]) {
     xs[0] = xs[1] = nullptr;
     if (ScalarOf<T>::cplx || !c->has_nl || !c->fuse_nl || !c->fuse_compact_gather || !c->nl.compact ||
-        c->nl.n_colors != 1)
+        c->nl.n_colors != 1 || nl_few_atoms(c->nl))
         return LYNX_OK;
     const long long ldw = ((long long)c->nl.n_pts + 3) & ~3LL;
     for (int i = 0; i < 2; ++i) {

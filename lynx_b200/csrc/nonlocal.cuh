@@ -3,7 +3,7 @@
 // :229-347 k-point; the reference GPU version uses atomicAdd in both halves,
 // src/operators/NonlocalProjector.cu:110-164,227-268).
 //
-//   gather : one CTA per (physical atom, block of NB columns) reduces all images
+//   gather : one CTA per (physical atom, block of columns) reduces all images
 //            of the atom in a fixed order:
 //              alpha[p][n] = Gamma_p * dV * sum_img e^{-i k.R_img} sum_g chi_img[g,p] psi[gpos[g], n]
 //            accumulated in the precision of the data (FP64 or FP32).
@@ -44,90 +44,189 @@ __device__ __forceinline__ double acc_phase(double v, double, double) { return v
 __device__ __forceinline__ double2 acc_phase(double2 v, double re, double im) {
     return make_double2(v.x * re - v.y * im, v.x * im + v.y * re);
 }
-
-constexpr int kGatherTile = 64;  // grid points per shared-memory tile
-
-// Accumulation type of the gather: FP64 for FP64 data, the data's own precision for FP32
-// data (a sum over one atom's sphere, ~10^3 terms).
-template <typename T> struct GAccOf { using type = T; };
-template <> struct GAccOf<double> { using type = double; };
 __device__ __forceinline__ float2 acc_phase(float2 v, double re, double im) {
     return make_float2((float)(v.x * re - v.y * im), (float)(v.x * im + v.y * re));
 }
 __device__ __forceinline__ float acc_phase(float v, double, double) { return v; }
 
-// gather: CTA = (atom, NB columns), 256 threads; thread = (column n, projector group jq),
-// projectors jq, jq+8, jq+16, ... (up to PJ of them).  The gathered x tile is staged in
-// shared memory with lanes along the grid points (coalesced loads).
-template <typename T, int NB, int PJ>
+__device__ __forceinline__ float shfl_x(float v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
+__device__ __forceinline__ double shfl_x(double v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
+__device__ __forceinline__ float2 shfl_x(float2 v, int o) { return make_float2(shfl_x(v.x, o), shfl_x(v.y, o)); }
+__device__ __forceinline__ double2 shfl_x(double2 v, int o) { return make_double2(shfl_x(v.x, o), shfl_x(v.y, o)); }
+
+// Sums M values over the 32 lanes of a warp by folding: in each of the five rounds a lane keeps one
+// half of its values and sends the other to its partner, so the whole takes about M shuffles
+// instead of 5 M.  Afterwards slot i of a lane holds the total of value fold_index(i, lane), or
+// nothing (-1).  The order of the additions is fixed.
+template <int M, int OFF, typename A, int N>
+__device__ __forceinline__ void warp_fold(A (&v)[N], int lane) {
+    if constexpr (OFF > 0) {
+        constexpr int H = (M + 1) / 2;
+        const bool up = (lane & OFF) != 0;
+#pragma unroll
+        for (int i = 0; i < H; ++i) {
+            const A lo = v[i], hi = (i + H < M) ? v[i + H] : vzero(A());
+            const A send = up ? lo : hi, keep = up ? hi : lo;
+            v[i] = vadd(keep, shfl_x(send, OFF));
+        }
+        warp_fold<H, OFF / 2>(v, lane);
+    }
+}
+template <int M, int OFF>
+__device__ __forceinline__ int fold_index(int i, int lane) {
+    if constexpr (OFF == 0) {
+        return i;
+    } else {
+        constexpr int H = (M + 1) / 2;
+        int j = fold_index<H, OFF / 2>(i, lane);
+        if (j < 0) return -1;
+        j += (lane & OFF) ? H : 0;
+        return j < M ? j : -1;
+    }
+}
+template <int M, int R>
+constexpr int fold_slots() {  // values left per lane after R rounds
+    if constexpr (R == 0) return M;
+    else return fold_slots<(M + 1) / 2, R - 1>();
+}
+
+// Gather for few atoms, with the lanes of a warp along the sphere points.  A CTA owns one atom and NC
+// columns; its eight warps take the atom's steps of 32 points in turn.  A lane loads its point's NP
+// projector values and NC values of x (both coalesced along the points) and keeps the NC x NP sums in
+// registers, so there is no staging, no barrier and no chain between steps: many loads are in flight
+// even when an atom has few points and few columns.  The sums over the lanes are folded, and the
+// warps are added in shared memory in a fixed order.  Complex data: the sums of one image, times the
+// image's phase, are added up per image.
+//
+// APPLY: the same CTA then adds the projectors' term, out[g] += scale * sum_j chi[j, g] alpha[j], at
+// its atom's points (j in order from zero, the order of the scatter kernels, so bitwise their
+// result).  Only when no grid point lies in two spheres: then every point has one writer.  alpha
+// does not leave the CTA.
+template <typename T, int NP, int NC, bool APPLY>
 __global__ void __launch_bounds__(256)
-    nl_gather_kernel(const T* __restrict__ x, long long ld, int ncol, int ncolp, NLView tab,
-                     T* __restrict__ alpha, double dV) {
+    nl_atom_kernel(const T* __restrict__ x, long long ld, int ncol, int ncolp, NLView tab, T* __restrict__ alpha,
+                   double dV, T* __restrict__ out, long long ldo, typename ScalarOf<T>::type scale) {
     using S = typename ScalarOf<T>::type;
-    using A = typename GAccOf<T>::type;
-    constexpr int G = kGatherTile;
-    constexpr int NBP = NB + 1;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    T* xs = reinterpret_cast<T*>(smraw);                          // G x NBP
-    S* cs = reinterpret_cast<S*>(smraw + sizeof(T) * G * NBP);    // G x np
+    constexpr int M = NP * NC;
+    __shared__ T red[8][M];
+    __shared__ T al[M];
     const S* chi = reinterpret_cast<const S*>(tab.chi);
-    const int a = blockIdx.x;
-    const int n0 = blockIdx.y * NB;
+    const int a = blockIdx.y;
     const int np = tab.atom_nproj[a];
+    if (np == 0) return;
     const int poff = tab.atom_poff[a];
-    const int tid = threadIdx.x;
-    const int n = tid % NB;
-    const int jq = tid / NB;
-    constexpr int JG = 256 / NB;  // projector groups
-    A acc[PJ];
+    const int i0 = tab.atom_img_ptr[a], i1 = tab.atom_img_ptr[a + 1];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int n0 = blockIdx.x * NC;
+    T acc[M];  // [projector][column]
 #pragma unroll
-    for (int m = 0; m < PJ; ++m) acc[m] = vzero(A());
-    for (int ii = tab.atom_img_ptr[a]; ii < tab.atom_img_ptr[a + 1]; ++ii) {
-        const int im = tab.atom_img_list[ii];
-        const int ndc = tab.img_ndc[im];
-        const int* gp = tab.gpos + tab.img_goff[im];
-        const S* ch = chi + tab.img_chi_off[im];
-        A part[PJ];
+    for (int q = 0; q < M; ++q) acc[q] = vzero(T());
+    if (n0 < ncol) {
+        const T* xc[NC];
 #pragma unroll
-        for (int m = 0; m < PJ; ++m) part[m] = vzero(A());
-        for (int g0 = 0; g0 < ndc; g0 += G) {
-            const int gl = min(G, ndc - g0);
-            __syncthreads();
-            for (int e = tid; e < G * NB; e += 256) {
-                const int g = e % G, c = e / G;
-                T v = vzero(T());
-                if (g < gl && n0 + c < ncol) v = x[(long long)gp[g0 + g] + (long long)(n0 + c) * ld];
-                xs[g * NBP + c] = v;
+        for (int c = 0; c < NC; ++c) xc[c] = x + (long long)min(n0 + c, ncol - 1) * ld;
+        int q0 = 0;  // steps of the images before this one
+        for (int ii = i0; ii < i1; ++ii) {
+            const int im = tab.atom_img_list[ii];
+            const int ndc = tab.img_ndc[im];
+            const int nst = (ndc + 31) >> 5;
+            const int* gp = tab.gpos + tab.img_goff[im];
+            const S* ch = chi + tab.img_chi_off[im];
+            T sum[ScalarOf<T>::cplx ? M : 1];
+            if constexpr (ScalarOf<T>::cplx) {
+#pragma unroll
+                for (int q = 0; q < M; ++q) sum[q] = vzero(T());
             }
-            for (int e = tid; e < G * np; e += 256) {
-                const int g = e % G, j = e / G;
-                cs[g * np + j] = (g < gl) ? ch[(long long)j * ndc + g0 + g] : S(0);
-            }
-            __syncthreads();
-            for (int g = 0; g < gl; ++g) {
-                const T xv = xs[g * NBP + n];
+#pragma unroll 2
+            for (int s = (w - q0) & 7; s < nst; s += 8) {
+                const int g = 32 * s + lane;
+                const bool ok = g < ndc;
+                const int gc = ok ? g : ndc - 1;
+                const long long o = gp[gc];
+                T xv[NC];
 #pragma unroll
-                for (int m = 0; m < PJ; ++m) {
-                    const int j = jq + m * JG;
-                    if (j < np) part[m] = fmac(part[m], (S)cs[g * np + j], xv);
+                for (int c = 0; c < NC; ++c) {
+                    xv[c] = xc[c][o];
+                    if (!ok) xv[c] = vzero(T());
+                }
+#pragma unroll
+                for (int j = 0; j < NP; ++j) {
+                    const S cv = ch[(long long)min(j, np - 1) * ndc + gc];
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        if constexpr (ScalarOf<T>::cplx) sum[j * NC + c] = fmac(sum[j * NC + c], cv, xv[c]);
+                        else acc[j * NC + c] = fmac(acc[j * NC + c], cv, xv[c]);
+                    }
                 }
             }
-        }
+            q0 += nst;
+            if constexpr (ScalarOf<T>::cplx) {
+                const double re = tab.img_phase[2 * im], ph = tab.img_phase[2 * im + 1];
 #pragma unroll
-        for (int m = 0; m < PJ; ++m)
-            acc[m] = vadd(acc[m], acc_phase(part[m], tab.img_phase[2 * im], tab.img_phase[2 * im + 1]));
+                for (int q = 0; q < M; ++q) acc[q] = vadd(acc[q], acc_phase(sum[q], re, ph));
+            }
+        }
+        warp_fold<M, 16>(acc, lane);
     }
 #pragma unroll
-    for (int m = 0; m < PJ; ++m) {
-        const int j = jq + m * JG;
-        if (j < np) {
-            // Gamma dV as an FP32 (hi, lo) pair: a single rounded float would scale the projector's
-            // channel by a fixed 1 + O(6e-8) and shift every Ritz value alike
-            const double gd = tab.gamma[poff + j] * dV;
-            const S hi = (S)gd;
-            T v = vscale(hi, acc[m]);
-            if (sizeof(S) == sizeof(float)) v = fmac(v, (S)(gd - (double)hi), acc[m]);
-            alpha[(long long)(poff + j) * ncolp + n0 + n] = v;
+    for (int i = 0; i < fold_slots<M, 5>(); ++i) {
+        const int q = fold_index<M, 16>(i, lane);
+        if (q >= 0) red[w][q] = acc[i];
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < np * NC; q += 256) {
+        const int j = q / NC, n = n0 + q % NC;
+        T t = red[0][q];
+#pragma unroll
+        for (int p = 1; p < 8; ++p) t = vadd(t, red[p][q]);
+        // Gamma dV as an FP32 (hi, lo) pair: a single rounded float would scale the projector's
+        // channel by a fixed 1 + O(6e-8) and shift every Ritz value alike
+        const double gd = tab.gamma[poff + j] * dV;
+        const S hi = (S)gd;
+        T v = vscale(hi, t);
+        if (sizeof(S) == sizeof(float)) v = fmac(v, (S)(gd - (double)hi), t);
+        if constexpr (APPLY) al[q] = v;
+        else if (n < ncolp) alpha[(long long)(poff + j) * ncolp + n] = n < ncol ? v : vzero(T());
+    }
+    if constexpr (APPLY) {
+        __syncthreads();
+        int q0 = 0;
+        for (int ii = i0; ii < i1; ++ii) {
+            const int im = tab.atom_img_list[ii];
+            const int ndc = tab.img_ndc[im];
+            const int nst = (ndc + 31) >> 5;
+            const int* gp = tab.gpos + tab.img_goff[im];
+            const S* ch = chi + tab.img_chi_off[im];
+            for (int s = (w - q0) & 7; s < nst; s += 8) {
+                const int g = 32 * s + lane;
+                if (g >= ndc) break;
+                T* o = out + gp[g];
+                T old[NC], v[NC];
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    old[c] = o[(long long)min(n0 + c, ncol - 1) * ldo];
+                    v[c] = vzero(T());
+                }
+#pragma unroll
+                for (int j = 0; j < NP; ++j) {
+                    if (j < np) {
+                        const S cv = ch[(long long)j * ndc + g];
+#pragma unroll
+                        for (int c = 0; c < NC; ++c) v[c] = fmac(v[c], cv, al[j * NC + c]);
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    if constexpr (ScalarOf<T>::cplx) {  // conj of the gather phase: e^{+i k.R_img}
+                        T ph;
+                        ph.x = (S)tab.img_phase[2 * im];
+                        ph.y = -(S)tab.img_phase[2 * im + 1];
+                        v[c] = pmul(v[c], ph);
+                    }
+                    if (n0 + c < ncol) o[(long long)(n0 + c) * ldo] = fmac(old[c], scale, v[c]);
+                }
+            }
+            q0 += nst;
         }
     }
 }

@@ -70,39 +70,60 @@ int gather2_dispatch(const NLDev& nl, const T* x, long long ld, int ncol, T* alp
 }
 }  // namespace
 
+namespace {
+// One CTA per (atom, NC columns).  NC x NP sums per lane fit the registers.
+template <typename T, bool APPLY>
+int launch_atom_kernel(const NLDev& nl, const T* x, long long ld, int ncol, T* alpha, int ncolp, double dV, T* out,
+                       long long ldo, typename ScalarOf<T>::type scale, cudaStream_t st) {
+    auto go = [&](auto kern, int nc) {
+        dim3 grid(((APPLY ? ncol : ncolp) + nc - 1) / nc, nl.n_atom);
+        kern<<<grid, 256, 0, st>>>(x, ld, ncol, ncolp, make_view<T>(nl), alpha, dV, out, ldo, scale);
+    };
+    constexpr int NC = std::is_same<T, float>::value ? 4 : std::is_same<T, double>::value ? 2 : 1;
+    constexpr int NC32 = NC >= 2 ? NC / 2 : 1;
+    if (nl.max_np <= 4) go(nl_atom_kernel<T, 4, NC, APPLY>, NC);
+    else if (nl.max_np <= 9) go(nl_atom_kernel<T, 9, NC, APPLY>, NC);
+    else if (nl.max_np <= 18) go(nl_atom_kernel<T, 18, NC, APPLY>, NC);
+    else go(nl_atom_kernel<T, 32, NC32, APPLY>, NC32);
+    count_launch();
+    return launch_status("nonlocal atom kernel");
+}
+}  // namespace
+
+bool nl_few_atoms(const NLDev& nl) { return nl.n_atom < kNLFewAtoms; }
+
 template <typename T>
 int launch_nl_gather(const NLDev& nl, const T* x, long long ld, int ncol, T* alpha, int ncolp, double dV,
                      cudaStream_t st) {
-    using S = typename ScalarOf<T>::type;
-    constexpr int NB = 32;  // columns per CTA; 8 projector groups of 256 threads
-    static_assert(kNLColBlock % 16 == 0 && NB % kNLColBlock == 0 || kNLColBlock % NB == 0, "column blocks");
     if (nl.n_atom == 0 || ncol <= 0) return LYNX_OK;
-    if constexpr (kReal<T>) {
-        if (nl.max_np <= 32) return gather2_dispatch<T>(nl, x, ld, ncol, alpha, ncolp, dV, st);
-    }
-    const int pj = (nl.max_np + 7) / 8;
-    if (pj > 4) {
+    if (nl.max_np > 32) {
         set_error("%d projectors per atom exceed the gather kernel's limit of 32", nl.max_np);
         return LYNX_ERR_UNSUPPORTED;
     }
-    const size_t smem = sizeof(T) * kGatherTile * (NB + 1) + sizeof(S) * nl.max_np * kGatherTile;
-    dim3 grid(nl.n_atom, (ncol + NB - 1) / NB);
-    auto go = [&](auto kern) {
-        smem_cap(kern, smem);
-        kern<<<grid, 256, smem, st>>>(x, ld, ncol, ncolp, make_view<T>(nl), alpha, dV);
-    };
-    if (pj <= 1) go(nl_gather_kernel<T, NB, 1>);
-    else if (pj == 2) go(nl_gather_kernel<T, NB, 2>);
-    else if (pj == 3) go(nl_gather_kernel<T, NB, 3>);
-    else go(nl_gather_kernel<T, NB, 4>);
-    count_launch();
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) {
-        set_error("nonlocal gather launch failed: %s", cudaGetErrorString(e));
-        return LYNX_ERR_CUDA;
+    if constexpr (kReal<T>) {
+        if (!nl_few_atoms(nl)) return gather2_dispatch<T>(nl, x, ld, ncol, alpha, ncolp, dV, st);
     }
-    return LYNX_OK;
+    return launch_atom_kernel<T, false>(nl, x, ld, ncol, alpha, ncolp, dV, nullptr, 0, 0, st);
 }
+
+template <typename T>
+int launch_nl_apply(const NLDev& nl, const T* x, long long ld, T* out, long long ldo, int ncol, double dV,
+                    typename ScalarOf<T>::type scale, cudaStream_t st) {
+    if (nl.n_atom == 0 || ncol <= 0) return LYNX_OK;
+    if (!nl.compact || nl.max_np > 32) {
+        set_error("the one-kernel nonlocal apply needs disjoint projector spheres and at most 32 projectors");
+        return LYNX_ERR_UNSUPPORTED;
+    }
+    return launch_atom_kernel<T, true>(nl, x, ld, ncol, nullptr, 0, dV, out, ldo, scale, st);
+}
+template int launch_nl_apply<double>(const NLDev&, const double*, long long, double*, long long, int, double, double,
+                                     cudaStream_t);
+template int launch_nl_apply<float>(const NLDev&, const float*, long long, float*, long long, int, double, float,
+                                    cudaStream_t);
+template int launch_nl_apply<double2>(const NLDev&, const double2*, long long, double2*, long long, int, double, double,
+                                      cudaStream_t);
+template int launch_nl_apply<float2>(const NLDev&, const float2*, long long, float2*, long long, int, double, float,
+                                     cudaStream_t);
 
 template <typename T, typename S>
 int launch_nl_scatter(const NLDev& nl, T* out, long long ld, int ncol, const T* alpha, int ncolp, S scale,

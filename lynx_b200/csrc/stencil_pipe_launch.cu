@@ -31,6 +31,8 @@ template <typename T> struct NumShapes { static constexpr int value = 1; };
 template <> struct NumShapes<float> { static constexpr int value = 4; };
 template <> struct NumShapes<double> { static constexpr int value = 4; };
 constexpr int kTunedR = 6;  // FD order 12
+constexpr int kFewCtas = 2 * 148;  // below this many CTAs, bands and z chunks are made shorter
+constexpr int kMinChunk = 4;       // planes of the shortest z chunk
 
 struct ShapeRT {
     int RX, RY, MAXT;
@@ -161,7 +163,11 @@ int launch_cheb_pipe(const StencilGeom& g, int nxp, const T* x, long long ldx, c
     TYT = std::min(TYT, (MT - 32) / P2);
     TYT = std::min(TYT, (g.ny + RY - 1) / RY);
     {
-        const int nb = std::min(g.ny, (g.ny + TYT * RY - 1) / (TYT * RY) + extra_bands);
+        int nb = std::min(g.ny, (g.ny + TYT * RY - 1) / (TYT * RY) + extra_bands);
+        // Few columns on a small grid: shorter bands as well as z chunks, so that there is a CTA for
+        // every SM (a CTA's time is its planes times the latency of one plane, not its points).
+        nb = std::max(nb, std::min((g.ny + RY - 1) / RY / 2, (kFewCtas + ncol * (g.nz / kMinChunk) - 1) /
+                                                           std::max(1, ncol * (g.nz / kMinChunk))));
         const int ty_bal = (g.ny + nb - 1) / nb;
         TYT = std::max(1, std::min(TYT, (ty_bal + RY - 1) / RY));
     }
@@ -183,6 +189,7 @@ int launch_cheb_pipe(const StencilGeom& g, int nxp, const T* x, long long ldx, c
     const int nbands = (g.ny + G.TY - 1) / G.TY;
     const long long base = (long long)nbands * ncol;
     int nzch = (int)std::min<long long>((600 + base - 1) / base, std::max(1, g.nz / (4 * R)));
+    if (base * nzch < kFewCtas) nzch = (int)std::min<long long>((kFewCtas + base - 1) / base, g.nz / kMinChunk);
     nzch = std::max(1, nzch);
     G.zchunk = (g.nz + nzch - 1) / nzch;
     nzch = (g.nz + G.zchunk - 1) / G.zchunk;
