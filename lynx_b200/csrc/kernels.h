@@ -30,9 +30,18 @@ struct NonOrthGeom {
 };
 // out += a * (-1/2) * (mixed-derivative part of Lap x); gy, gz: scratch blocks like x (column
 // stride ldg).  nonorth.cu.
+// have_grads: gy and gz already hold the first derivatives of x (launch_direct_step).
 template <typename T>
 int launch_nonorth_terms(const NonOrthGeom& g, int nxp, const T* x, long long ldx, T* gy, T* gz, long long ldg, T* out,
-                         long long ldout, int ncol, double a, const T* phl, const T* phr, cudaStream_t st);
+                         long long ldout, int ncol, double a, const T* phl, const T* phr, cudaStream_t st,
+                         bool have_grads = false);
+// The Chebyshev step of small problems, one thread per point (stencil_direct.cu, FD order 12, any
+// row pitch and alignment).  ng (may be null): also write the first derivatives of x along y and z
+// to gy and gz (column stride ldg).
+template <typename T, typename S>
+int launch_direct_step(const StencilGeom& g, int nxp, const T* x, long long ldx, const T* xold, long long ldo, T* out,
+                       long long ldout, const S* V, int ncol, double a, double b, double d, const T* phl,
+                       const T* phr, const NonOrthGeom* ng, T* gy, T* gz, long long ldg, cudaStream_t st);
 
 // out = a*(-0.5*Lap x + V.*x) + b*x + d*xold over ncol columns (xold may be null when d == 0).
 // phl/phr: per-direction ghost multipliers (3 values of T each).
@@ -131,6 +140,18 @@ int launch_rot_i8(const float* Y, long long ldy, long long rows, int nx, int nxp
 template <typename T>
 int launch_density(const T* psi, long long ld, long long nd, int ncol, const double* w, double* rho, bool accumulate,
                    cudaStream_t st);
+
+// Rayleigh-Ritz step of few states (small_rr.cu): products in FP64, one CTA for the subspace algebra.
+// Y, HY: blocks of n columns, ld >= rows elements apart, rows of nxp with nx valid points (pads
+// zero); Ms, Hs: n x n scratch of the wide type (double / double2), psi: nd points per column, stride
+// ldp.  info as in rr_alloc_small.  work: small_rr_work_bytes.
+constexpr int kSmallRRMax = 40;
+bool small_rr_supported(int n);
+size_t small_rr_work_bytes(long long rows, int n, size_t wide);
+template <typename T>
+int launch_small_rr(const T* Y, const T* HY, long long ld, long long rows, int nx, int nxp, long long nd, int n,
+                    double dV, void* work, void* Ms, void* Hs, double* eig, int* info, void* psi, long long ldp,
+                    cudaStream_t st);
 
 // Effective potential (veff.cu), FP64 fields of nx ny nz points, x fastest.
 struct GradGeom {

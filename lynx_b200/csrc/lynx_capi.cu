@@ -793,6 +793,13 @@ int stencil_time_add(lynx_ctx* c) {
     return LYNX_OK;
 }
 
+// The one-thread-per-point kernel (stencil_direct.cu) takes complex blocks, and real ones that are
+// small enough to be bound by latency (both sides measured: see that file).
+constexpr long long kDirectRealBytes = 1250000;
+template <typename T> bool direct_step_pays(long long nd, int ncol) {
+    return ScalarOf<T>::cplx || nd * ncol * (long long)sizeof(T) <= kDirectRealBytes;
+}
+
 // One Chebyshev step out = a H x + b x + d xold (H with the nonlocal term when tables are set).
 // With the fused nonlocal path, xs_in (optional) is the compact sphere-point copy of x written
 // by the previous step, and xs_out (optional) receives the compact copy of out; *xs_written
@@ -822,6 +829,7 @@ int cheb_step(lynx_ctx* c, int nxp, const T* x, long long ldx, const T* xold, lo
                       c->nl.n_colors == 1 && geom(c).R == 6 && c->bc[0] == LYNX_BC_PERIODIC &&
                       c->bc[1] == LYNX_BC_PERIODIC && c->bc[2] == LYNX_BC_PERIODIC;
     const long long ldw = ((long long)c->nl.n_pts + 3) & ~3LL;  // compact column stride
+    const bool direct = ScalarOf<T>::cplx || (!fuse && c->force_shape < 0 && direct_step_pays<T>(c->Nd, ncol));
     const NLDev* nl = nullptr;
     if (c->has_nl) LYNX_TRY(nl_for(c, nxp, &nl));
     if (c->has_nl && !few) {
@@ -835,9 +843,26 @@ int cheb_step(lynx_ctx* c, int nxp, const T* x, long long ldx, const T* xold, lo
             LYNX_TRY(launch_nl_gather<T>(*nl, x, ldx, ncol, c->alpha.as<T>(), ncolp, c->dV, c->stream));
         }
     }
-    if (pipe_ok) {
-        if (!c->errflag.p) LYNX_TRY(ensure_zeroed(c, c->errflag, sizeof(int)));
-        if constexpr (!ScalarOf<T>::cplx) {
+    const long long ldg = (long long)nxp * c->ny * c->nz;
+    NonOrthGeom ng{};
+    T *gy = nullptr, *gz = nullptr;
+    if (!c->orth) {
+        // mixed-derivative terms of a non-orthogonal cell, from two first-derivative blocks
+        for (int i = 0; i < 2; ++i) LYNX_TRY(c->gradbuf[i].ensure(sizeof(T) * (size_t)ldg * ncol));
+        gy = c->gradbuf[0].as<T>();
+        gz = c->gradbuf[1].as<T>();
+        ng = NonOrthGeom{c->nx, c->ny, c->nz, geom(c).R, c->D1y.data(), c->D1z.data(), c->D2xy.data(), c->D2xz.data(),
+                         c->D2yz.data()};
+    }
+    if (direct) {
+        if (c->time_stencil) LYNX_CUDA_TRY(cudaEventRecord(c->kt[0], c->stream));
+        LYNX_TRY(launch_direct_step<T, S>(geom(c), nxp, x, ldx, xold, ldo, out, ldout, V, ncol, a, b, d, phl, phr,
+                                          c->orth ? nullptr : &ng, gy, gz, ldg, c->stream));
+        if (c->time_stencil) LYNX_TRY(stencil_time_add(c));
+    }
+    if constexpr (!ScalarOf<T>::cplx) {
+        if (!direct && pipe_ok) {
+            if (!c->errflag.p) LYNX_TRY(ensure_zeroed(c, c->errflag, sizeof(int)));
             if (fuse) {
                 const lynx_ctx::NLMap* nm = nullptr;
                 LYNX_TRY(nl_map_for(c, nxp, &nm));
@@ -852,22 +877,18 @@ int cheb_step(lynx_ctx* c, int nxp, const T* x, long long ldx, const T* xold, lo
                 if (xs_written) *xs_written = (xs_out != nullptr);
                 return LYNX_OK;
             }
+            if (c->time_stencil) LYNX_CUDA_TRY(cudaEventRecord(c->kt[0], c->stream));
+            LYNX_TRY(pipe_launch_tuned<T, S>(c, nxp, x, ldx, xold, ldo, out, ldout, V, ncol, a, b, d, phl, phr,
+                                             nullptr));
+            if (c->time_stencil) LYNX_TRY(stencil_time_add(c));
+        } else if (!direct) {
+            LYNX_TRY(launch_cheb_step<T, S>(geom(c), x, ldx, xold, ldo, out, ldout, V, ncol, a, b, d, phl, phr,
+                                            c->stream));
         }
-        if (c->time_stencil) LYNX_CUDA_TRY(cudaEventRecord(c->kt[0], c->stream));
-        LYNX_TRY(pipe_launch_tuned<T, S>(c, nxp, x, ldx, xold, ldo, out, ldout, V, ncol, a, b, d, phl, phr, nullptr));
-        if (c->time_stencil) LYNX_TRY(stencil_time_add(c));
-    } else {
-        LYNX_TRY(launch_cheb_step<T, S>(geom(c), x, ldx, xold, ldo, out, ldout, V, ncol, a, b, d, phl, phr, c->stream));
     }
-    if (!c->orth) {
-        // mixed-derivative terms of a non-orthogonal cell, from two first-derivative blocks
-        const long long ldg = (long long)nxp * c->ny * c->nz;
-        for (int i = 0; i < 2; ++i) LYNX_TRY(c->gradbuf[i].ensure(sizeof(T) * (size_t)ldg * ncol));
-        NonOrthGeom ng{c->nx, c->ny, c->nz, geom(c).R, c->D1y.data(), c->D1z.data(), c->D2xy.data(), c->D2xz.data(),
-                       c->D2yz.data()};
-        LYNX_TRY(launch_nonorth_terms<T>(ng, nxp, x, ldx, c->gradbuf[0].as<T>(), c->gradbuf[1].as<T>(), ldg, out, ldout,
-                                         ncol, a, phl, phr, c->stream));
-    }
+    if (!c->orth)
+        LYNX_TRY(launch_nonorth_terms<T>(ng, nxp, x, ldx, gy, gz, ldg, out, ldout, ncol, a, phl, phr, c->stream,
+                                         direct));
     if (few) LYNX_TRY(launch_nl_apply<T>(*nl, x, ldx, out, ldout, ncol, c->dV, (S)a, c->stream));
     else if (c->has_nl)
         LYNX_TRY(launch_nl_scatter<T, S>(*nl, out, ldout, ncol, c->alpha.as<T>(), ncolp, (S)a, c->stream));
@@ -1309,6 +1330,19 @@ int rayleigh_ritz(lynx_ctx* c, const double2* Y, long long ldY, const double2* H
     return rayleigh_ritz_cplx(c, Y, ldY, HY, ldH, psi, ldp, N, eig);
 }
 
+// Few states: products, subspace algebra and rotation in four launches (small_rr.cu).
+template <typename T>
+int rayleigh_ritz_small(lynx_ctx* c, const T* Y, const T* HY, long long ldb, int nxp, void* psi, long long ldp, int N,
+                        double* eig_host) {
+    const size_t wide = ScalarOf<T>::cplx ? sizeof(double2) : sizeof(double);
+    const long long rows = (long long)nxp * c->ny * c->nz;  // pad elements are zero
+    LYNX_TRY(rr_alloc_small(c, N, wide));
+    LYNX_TRY(c->gwork.ensure(small_rr_work_bytes(rows, N, wide)));
+    LYNX_TRY(launch_small_rr<T>(Y, HY, ldb, rows, c->nx, nxp, c->Nd, N, c->dV, c->gwork.p, c->Ms.p, c->Hs.p,
+                                c->eigd.as<double>(), c->info.as<int>(), psi, ldp, c->stream));
+    return finish_rr(c, N, eig_host);
+}
+
 // ---------------------------------------------------------------------------
 // CheFSI pass.  T64 = FP64 storage type (double / double2), T32 = FP32 (float / float2).
 // ---------------------------------------------------------------------------
@@ -1331,7 +1365,9 @@ int solve_impl(lynx_ctx* c, T64* psi, double* eig, const double* veff, int N, in
     if (precision == LYNX_PREC_FP64) {
         T64 *Y = nullptr, *HY = nullptr;
         LYNX_TRY(run_filter64<T64>(c, psi, ldp, veff, N, lc, emin, emax, degree, use_k, true, &Y, &HY, &ldb, &nxp));
-        if (nxp == c->nx) {
+        if (small_rr_supported(N)) {
+            LYNX_TRY(rayleigh_ritz_small<T64>(c, Y, HY, ldb, nxp, psi, ldp, N, eig));
+        } else if (nxp == c->nx) {
             LYNX_TRY(rayleigh_ritz(c, Y, ldb, HY, ldb, psi, ldp, N, eig));
         } else {
             LYNX_TRY(c->cvt[0].ensure(blk64));
@@ -1344,6 +1380,12 @@ int solve_impl(lynx_ctx* c, T64* psi, double* eig, const double* veff, int N, in
         T32 *Y = nullptr, *HY = nullptr;
         LYNX_TRY(run_filter32<T32, T64>(c, psi, ldp, veff, N, lc, emin, emax, degree, use_k, true, &Y, &HY, &ldb,
                                         &nxp));
+        if (small_rr_supported(N) && !c->no_tc_gram) {
+            LYNX_TRY(rayleigh_ritz_small<T32>(c, Y, HY, ldb, nxp, psi, ldp, N, eig));
+            LYNX_TRY(check_errflag(c));
+            if (lc_out) *lc_out = eig[N - 1] + 0.1;
+            return LYNX_OK;
+        }
         if constexpr (std::is_same<T32, float>::value) {
             if (pipe_capable<float>(c->nx) && !c->no_tc_gram) {
                 LYNX_TRY(rayleigh_ritz_mixed_real(c, Y, HY, ldb, nxp, reinterpret_cast<double*>(psi), ldp, N, eig));

@@ -111,7 +111,8 @@ __global__ void __launch_bounds__(256)
 
 template <typename T>
 int launch_nonorth_terms(const NonOrthGeom& g, int nxp, const T* x, long long ldx, T* gy, T* gz, long long ldg, T* out,
-                         long long ldout, int ncol, double a, const T* phl, const T* phr, cudaStream_t st) {
+                         long long ldout, int ncol, double a, const T* phl, const T* phr, cudaStream_t st,
+                         bool have_grads) {
     using S = typename ScalarOf<T>::type;
     if (g.R < 1 || g.R > 8) {
         set_error("FD half-width %d outside the supported range 1..8", g.R);
@@ -142,9 +143,9 @@ int launch_nonorth_terms(const NonOrthGeom& g, int nxp, const T* x, long long ld
     }
     const long long np = (long long)g.nx * g.ny * g.nz;
     dim3 grid((unsigned)((np + 255) / 256), ncol);
-    nonorth_grad_kernel<T><<<grid, 256, 0, st>>>(x, ldx, gy, gz, ldg, A);
+    if (!have_grads) nonorth_grad_kernel<T><<<grid, 256, 0, st>>>(x, ldx, gy, gz, ldg, A);
     nonorth_mixed_kernel<T><<<grid, 256, 0, st>>>(gy, gz, ldg, out, ldout, (S)(-0.5 * a), A);
-    count_launch(2);
+    count_launch(have_grads ? 1 : 2);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         set_error("non-orthogonal stencil launch failed: %s", cudaGetErrorString(e));
@@ -154,15 +155,15 @@ int launch_nonorth_terms(const NonOrthGeom& g, int nxp, const T* x, long long ld
 }
 
 template int launch_nonorth_terms<double>(const NonOrthGeom&, int, const double*, long long, double*, double*, long long,
-                                          double*, long long, int, double, const double*, const double*, cudaStream_t);
+                                          double*, long long, int, double, const double*, const double*, cudaStream_t, bool);
 template int launch_nonorth_terms<float>(const NonOrthGeom&, int, const float*, long long, float*, float*, long long,
-                                         float*, long long, int, double, const float*, const float*, cudaStream_t);
+                                         float*, long long, int, double, const float*, const float*, cudaStream_t, bool);
 template int launch_nonorth_terms<double2>(const NonOrthGeom&, int, const double2*, long long, double2*, double2*,
                                            long long, double2*, long long, int, double, const double2*, const double2*,
-                                           cudaStream_t);
+                                           cudaStream_t, bool);
 template int launch_nonorth_terms<float2>(const NonOrthGeom&, int, const float2*, long long, float2*, float2*,
                                           long long, float2*, long long, int, double, const float2*, const float2*,
-                                          cudaStream_t);
+                                          cudaStream_t, bool);
 
 }  // namespace lynxb
 

@@ -1,6 +1,5 @@
-// Launch-shape selection and template dispatch for the fused Chebyshev-step kernel.
-// Compiled once per value type (LYNX_STENCIL_TYPES selects real or complex) so the
-// instantiations build in parallel.
+// Launch-shape selection and template dispatch for the fused Chebyshev-step kernel (real data;
+// complex blocks: stencil_direct.cu).
 #include <algorithm>
 #include <cstdio>
 #include <type_traits>
@@ -13,7 +12,7 @@ namespace lynxb {
 
 namespace {
 
-template <typename T> constexpr int rows_per_thread() { return ScalarOf<T>::cplx ? 1 : 2; }
+template <typename T> constexpr int rows_per_thread() { return 2; }
 
 template <typename T, int R, int HK, bool XOLD>
 void launch_one(dim3 grid, int nthr, size_t smem, cudaStream_t st, const T* x, const T* xold, T* out,
@@ -130,20 +129,11 @@ int launch_cheb_step(const StencilGeom& g, const T* x, long long ldx, const T* x
     return LYNX_OK;
 }
 
-#if LYNX_STENCIL_TYPES == 0
 template int launch_cheb_step<double, double>(const StencilGeom&, const double*, long long, const double*,
                                               long long, double*, long long, const double*, int, double,
                                               double, double, const double*, const double*, cudaStream_t);
 template int launch_cheb_step<float, float>(const StencilGeom&, const float*, long long, const float*,
                                             long long, float*, long long, const float*, int, double, double,
                                             double, const float*, const float*, cudaStream_t);
-#else
-template int launch_cheb_step<double2, double>(const StencilGeom&, const double2*, long long, const double2*,
-                                               long long, double2*, long long, const double*, int, double,
-                                               double, double, const double2*, const double2*, cudaStream_t);
-template int launch_cheb_step<float2, float>(const StencilGeom&, const float2*, long long, const float2*,
-                                             long long, float2*, long long, const float*, int, double, double,
-                                             double, const float2*, const float2*, cudaStream_t);
-#endif
 
 }  // namespace lynxb

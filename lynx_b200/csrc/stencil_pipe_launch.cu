@@ -1,5 +1,5 @@
 // Launch-shape selection and template dispatch for the pipelined Chebyshev-step kernel.
-// LYNX_STENCIL_TYPES = 0: real (double, float); 1: complex (double2, float2).
+// Real data (complex blocks: stencil_direct.cu).
 #include <algorithm>
 #include <cstdio>
 #include <type_traits>
@@ -25,8 +25,6 @@ template <> struct PipeShapeAt<double, 0> { static constexpr int RX = 2, RY = 2,
 template <> struct PipeShapeAt<double, 1> { static constexpr int RX = 2, RY = 1, MAXT = 512; };
 template <> struct PipeShapeAt<double, 2> { static constexpr int RX = 2, RY = 1, MAXT = 640; };
 template <> struct PipeShapeAt<double, 3> { static constexpr int RX = 2, RY = 2, MAXT = 384; };
-template <> struct PipeShapeAt<float2, 0> { static constexpr int RX = 1, RY = 4, MAXT = 352; };
-template <> struct PipeShapeAt<double2, 0> { static constexpr int RX = 1, RY = 2, MAXT = 352; };
 template <typename T> struct NumShapes { static constexpr int value = 1; };
 template <> struct NumShapes<float> { static constexpr int value = 4; };
 template <> struct NumShapes<double> { static constexpr int value = 4; };
@@ -269,7 +267,6 @@ int launch_cheb_pipe(const StencilGeom& g, int nxp, const T* x, long long ldx, c
     return LYNX_OK;
 }
 
-#if LYNX_STENCIL_TYPES == 0
 template int launch_cheb_pipe<double, double>(const StencilGeom&, int, const double*, long long, const double*,
                                               long long, double*, long long, const double*, int, double, double,
                                               double, const double*, const double*, int*, cudaStream_t, int, const PipeNLHost*);
@@ -278,15 +275,5 @@ template int launch_cheb_pipe<float, float>(const StencilGeom&, int, const float
                                             const float*, const float*, int*, cudaStream_t, int, const PipeNLHost*);
 template int pipe_shape_count<double>(int);
 template int pipe_shape_count<float>(int);
-#else
-template int launch_cheb_pipe<double2, double>(const StencilGeom&, int, const double2*, long long, const double2*,
-                                               long long, double2*, long long, const double*, int, double, double,
-                                               double, const double2*, const double2*, int*, cudaStream_t, int, const PipeNLHost*);
-template int launch_cheb_pipe<float2, float>(const StencilGeom&, int, const float2*, long long, const float2*,
-                                             long long, float2*, long long, const float*, int, double, double,
-                                             double, const float2*, const float2*, int*, cudaStream_t, int, const PipeNLHost*);
-template int pipe_shape_count<double2>(int);
-template int pipe_shape_count<float2>(int);
-#endif
 
 }  // namespace lynxb

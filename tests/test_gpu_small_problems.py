@@ -1,0 +1,121 @@
+"""Kernels of small problems: the one-thread-per-point stencil, the one-kernel nonlocal apply of few
+atoms, and the four-launch Rayleigh-Ritz step of few states, against the numpy oracle, the pipelined
+stencil and dense linear algebra."""
+import numpy as np
+import pytest
+
+from helpers import si8_small
+from lynx_b200 import _lib
+from lynx_b200 import cell as C
+from lynx_b200 import pseudo as P
+from oracle import chefsi_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _oracle(cl, tab):
+    t = dict(img_atom=tab.img_atom, img_ndc=tab.img_ndc, img_shift=tab.img_shift, gpos=tab.gpos, chi=tab.chi,
+             gamma=tab.gamma, nproj=int(tab.atom_nproj[0]))
+    return O.Operator(cl.latvec, cl.shape, cl.fd_order, cl.orthogonal, t)
+
+
+def _cell(kind, shape):
+    if kind == "fcc":
+        cl, pos = C.fcc_si_primitive(shape[0])
+        cl.shape = shape
+        return cl, pos, C.synthetic_veff(cl, pos, noise=1e-3, seed=2)
+    cl, pos, V = si8_small(grid=shape)
+    return cl, pos, V
+
+
+# FP64: sums of about 60 terms of size ~40 |x| (coefficients / h^2): 60 * 2^-53 * 40 / |H x| < 1e-13.
+@pytest.mark.parametrize("kind,shape,ncol,kpt", [
+    ("si8", (20, 21, 22), 1, False), ("si8", (21, 20, 23), 3, False), ("si8", (20, 20, 20), 25, False),
+    ("si8", (20, 21, 22), 5, True), ("si8", (31, 33, 30), 2, True), ("fcc", (20, 20, 20), 4, False),
+    ("fcc", (17, 19, 18), 3, True)])
+@pytest.mark.parametrize("fd_order", [12, 8])
+def test_h_apply_of_small_blocks(synth_psp8, kind, shape, ncol, kpt, fd_order):
+    from lynx_b200 import solver
+    cl, pos, V = _cell(kind, shape)
+    cl.fd_order = fd_order
+    tab = P.nonlocal_tables(cl, pos, P.read_psp8(synth_psp8))
+    ctx = solver.Context(cl)
+    ctx.set_nonlocal(tab)
+    k = np.array([0.25, -0.125, 0.375]) * 2 * np.pi / cl.lengths
+    x = C.random_orbitals(ctx.nd, ncol, seed=3, complex_=kpt)
+    h = solver.Hamiltonian(ctx, V)
+    if kpt:
+        ctx.set_kpoint(k)
+        y = h.apply_kpt(x)
+    else:
+        y = h.apply(x)
+    want = _oracle(cl, tab).apply(x, V, kpt=k if kpt else None)
+    assert np.abs(y - want).max() < 1e-12 * np.abs(want).max()
+    ctx.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("shape,ncol", [((20, 21, 22), 7), ((24, 24, 24), 1), ((22, 24, 26), 17)])
+def test_direct_step_is_the_pipelined_one(synth_psp8, precision, shape, ncol):
+    """The same sums in the same order: bitwise the pipelined kernel's filter (forced by the launch
+    shape option)."""
+    from lynx_b200 import solver
+    cl, pos, V = _cell("si8", shape)
+    ctx = solver.Context(cl)
+    ctx.set_nonlocal(P.nonlocal_tables(cl, pos, P.read_psp8(synth_psp8)))
+    es = solver.EigenSolver(ctx, precision)
+    x = C.random_orbitals(ctx.nd, ncol, seed=4)
+    out = []
+    for forced in (0, 1):
+        ctx.set_option(_lib.OPT_STENCIL_SHAPE, forced)
+        out.append(es.chebyshev_filter(x, V, 25.0, -2.0, 70.0, degree=5))
+    assert np.array_equal(out[0], out[1])
+    ctx.close()
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 24, 39, 40, 41])
+@pytest.mark.parametrize("kpt", [False, True])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_rayleigh_ritz_of_few_states(synth_psp8, n, kpt, precision):
+    """One pass against dense linear algebra on the filtered block (n = 41: the library path).  FP64:
+    eps times the condition of the overlap (a degree-4 filter: below 1e4).  Mixed: the FP32 filter."""
+    from lynx_b200 import solver
+    cl, pos, V = _cell("si8", (18, 17, 20))
+    tab = P.nonlocal_tables(cl, pos, P.read_psp8(synth_psp8))
+    ctx = solver.Context(cl)
+    ctx.set_nonlocal(tab)
+    k = np.array([0.25, -0.125, 0.375]) * 2 * np.pi / cl.lengths if kpt else None
+    if kpt:
+        ctx.set_kpoint(k)
+    lo, hi = float(V.min()) - 1.0, ctx.max_eigval_half_lap + 8.0
+    x = C.random_orbitals(ctx.nd, n, seed=5, complex_=kpt)
+    es = solver.EigenSolver(ctx, precision)
+    psi, eig = (es.solve_kpt if kpt else es.solve)(x, V, 0.5 * (lo + hi), lo, hi, 4)
+    want, e_want, _ = O.solve(_oracle(cl, tab), x, V, 0.5 * (lo + hi), lo, hi, 4, kpt=k)
+    tol = 1e-11 if precision == "fp64" else 2e-5
+    assert np.all(np.diff(eig) >= 0)
+    assert np.abs(eig - e_want).max() < tol * np.abs(e_want).max()
+    s = psi.conj().T @ psi * cl.dV
+    assert np.abs(s - np.eye(n)).max() < (1e-11 if precision == "fp64" else 1e-5)
+    sv = np.linalg.svd(psi.conj().T @ want * cl.dV, compute_uv=False)
+    assert np.abs(sv - 1).max() < (1e-11 if precision == "fp64" else 1e-5)
+    ctx.close()
+
+
+@pytest.mark.parametrize("n", [4, 7])
+def test_degenerate_states(n):
+    """V = 0, no projectors, plane waves: the Ritz values of the cubic cell are degenerate in exact
+    groups; the rotations must still converge and leave an orthonormal block."""
+    from lynx_b200 import solver
+    cl = C.diamond_si(1, 18)[0]
+    ctx = solver.Context(cl)
+    g = np.arange(18) * 2 * np.pi / 18
+    zz, yy, xx = np.meshgrid(g, g, g, indexing="ij")
+    waves = [np.ones(18 ** 3)] + [f(t).ravel() for t in (xx, yy, zz) for f in (np.cos, np.sin)]
+    x = np.asfortranarray(np.stack(waves[:n], axis=1))
+    hi = ctx.max_eigval_half_lap + 1.0
+    psi, eig = solver.EigenSolver(ctx, "fp64").solve(x, np.zeros(ctx.nd), 0.5 * hi, -0.5, hi, 2)
+    e1 = O.Operator(cl.latvec, cl.shape).apply(x[:, 1:2], np.zeros(ctx.nd))[5, 0] / x[5, 1]
+    assert np.abs(eig - np.array([0.0] + [e1] * (n - 1))).max() < 1e-11
+    assert np.abs(psi.T @ psi * cl.dV - np.eye(n)).max() < 1e-11
+    ctx.close()
