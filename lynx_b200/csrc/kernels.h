@@ -270,22 +270,29 @@ int launch_nl_apply(const NLDev& nl, const T* x, long long ld, T* out, long long
 template <typename T, typename S>
 int launch_nl_scatter(const NLDev& nl, T* out, long long ld, int ncol, const T* alpha, int ncolp, S scale,
                       cudaStream_t st);
-// Nonlocal force of one direction and per-atom energy from projections without Gamma (alpha of
-// psi, beta of its derivative), occupations occ (device): see nonlocal.cuh.
+// Forces and stress (forces.cu): grid, host FD first-derivative coefficients (R + 1 per direction),
+// spacings, and for non-orthogonal cells ui = uvec^-1 and uvec (row-major).
+struct ForceGeom {
+    int nx, ny, nz, R;
+    bool orth;
+    const double* D1[3];
+    double h[3], ui[9], uvec[9];
+};
+// Per atom a: out[a][v] = scale * sum_n occ[n] sum_j Gamma_j Re(conj(alpha_j) beta_jv) and ea[a] = escale
+// * sum_n occ[n] sum_j Gamma_j |alpha_j|^2, with alpha = dV chi^T psi, beta_v the projections of the FD
+// derivatives along the three lattice directions (v < 3), or (stress) of the Cartesian derivatives
+// times the position relative to the image (img_pos, device), v = xx xy xz yy yz zz.  All device.
+size_t sphere_work_bytes(int n_atom, int ncol, bool stress);
 template <typename T>
-int launch_nl_force_reduce(const NLDev& nl, const T* alpha, const T* beta, int ncolp, int ncol, const double* occ,
-                           double spn, double efac, int dim, double* force, double* ea, cudaStream_t st);
-// First derivative along lattice direction dir (D1: R+1 host coefficients); nonorth.cu.
+int launch_sphere_terms(const NLDev& nl, const ForceGeom& g, const T* psi, long long ld, int ncol, const T* phl,
+                        const T* phr, const double* img_pos, const double* occ, double scale, double escale,
+                        double dV, bool stress, double* work, double* out, double* ea, cudaStream_t st);
+// out[v] = scale * sum_n occ[n] sum_r Re(conj(D_a psi_n) D_b psi_n), v = xx xy xz yy yz zz (Cartesian FD
+// gradients); phased: some ghost multiplier is not 1.
+size_t kinetic_work_bytes(const ForceGeom& g, int ncol, bool cplx);
 template <typename T>
-int launch_grad_dir(int nx, int ny, int nz, int nxp, int R, const double* D1, int dir, const T* x, long long ldx,
-                    T* g, long long ldg, int ncol, const T* phl, const T* phr, cudaStream_t st);
-// Stress helpers (nonorth.cu): in-place Cartesian mixing of three lattice-direction gradient
-// blocks of n elements (uinv: 3x3 row-major uvec^-1), and the six Voigt products per column.
-template <typename T>
-int launch_cart_mix(T* g0, T* g1, T* g2, long long n, const double* uinv, cudaStream_t st);
-template <typename T>
-int launch_dot6(const T* g0, const T* g1, const T* g2, long long nd, long long ld, int ncol, double* out,
-                cudaStream_t st);
+int launch_kinetic(const ForceGeom& g, const T* psi, long long ld, int ncol, const T* phl, const T* phr, bool phased,
+                   const double* occ, double scale, double* work, double* out, cudaStream_t st);
 // W[col * ldw + point] = (chi alpha)(point, col) on the compact point numbering (nl.compact).
 template <typename T>
 int launch_nl_expand(const NLDev& nl, T* W, long long ldw, int ncol, const T* alpha, int ncolp, cudaStream_t st);

@@ -327,7 +327,7 @@ struct lynx_ctx {
     DevBuf nlW;                    // compact (chi alpha) values, columns of ldw
     DevBuf xsbuf[2];               // compact sphere-point copies of consecutive filter blocks
     DevBuf gradbuf[2];             // first derivatives along y and z (non-orthogonal cells)
-    DevBuf fbeta, fwork, fones;    // nonlocal forces: derivative projections, occupations/results, ones
+    DevBuf fpart, fwork;           // forces, stress: partial sums; occupations, positions, results
     // Host-input pipelining: a copy stream, and for the duration of one host-pointer solve the
     // first column of every column block with the event that marks its arrival on the device.
     cudaStream_t copy_stream = nullptr;
@@ -336,11 +336,6 @@ struct lynx_ctx {
     std::map<int, NLDev> nl_layouts;
     std::vector<DevBuf> nl_layout_bufs;
     std::vector<int> h_gpos, h_pt_grid;  // host copies of the unpadded grid indices
-    // host copies for the stress: per-image offsets into gpos / chi, point counts, atoms; chi
-    std::vector<long long> h_img_goff, h_img_choff;
-    std::vector<int> h_img_ndc, h_img_atom, h_atom_nproj;
-    std::vector<double> h_chi;
-    DevBuf sbuf[4];  // stress: third gradient block, chi weighted by x, y, z relative positions
     // lynx_eigensolver_solve_density: the density request of the current pass
     struct DensityReq {
         bool on = false, done = false;
@@ -1708,10 +1703,8 @@ int lynx_destroy(lynx_ctx* c) {
     c->xsbuf[1].release();
     c->gradbuf[0].release();
     c->gradbuf[1].release();
-    c->fbeta.release();
+    c->fpart.release();
     c->fwork.release();
-    c->fones.release();
-    for (auto& b : c->sbuf) b.release();
     if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
     for (cudaEvent_t e : c->kt)
         if (e) cudaEventDestroy(e);
@@ -1984,12 +1977,6 @@ int lynx_set_nonlocal(lynx_ctx* c, int n_img, const int* img_atom, const int* im
     c->img_shift.assign(img_shift, img_shift + 3 * n_img);
     c->h_gpos.assign(gpos, gpos + tot);
     c->h_pt_grid = pt_grid;
-    c->h_img_goff = goff;
-    c->h_img_choff = choff;
-    c->h_img_ndc.assign(img_ndc, img_ndc + n_img);
-    c->h_img_atom.assign(img_atom, img_atom + n_img);
-    c->h_atom_nproj = nproj;
-    c->h_chi.assign(chi, chi + totchi);
     c->has_nl = true;
     return update_nl_phases(c);
 }
@@ -2317,8 +2304,16 @@ int noalloc_scratch(int device, void** out) {
 }
 }  // namespace
 
-// Nonlocal forces (src/physics/Forces.cpp:509-797): projections without Gamma of psi and of its
-// FD derivative along each lattice direction, reduced per atom with the occupations.
+static ForceGeom force_geom(const lynx_ctx* c) {
+    ForceGeom g{c->nx, c->ny, c->nz, c->R, c->orth, {c->D1x.data(), c->D1y.data(), c->D1z.data()},
+                {c->dx, c->dy, c->dz}, {}, {}};
+    std::copy(c->uvec, c->uvec + 9, g.uvec);
+    if (!c->orth) mat3_inverse(c->uvec, g.ui);  // Cartesian gradients: D_cart = uvec^-1 D_lattice
+    return g;
+}
+
+// Nonlocal forces (src/physics/Forces.cpp:509-797): projections of psi and of its FD derivative along
+// each lattice direction, reduced per atom with the occupations (forces.cu).
 template <typename T>
 int nonlocal_force_impl(lynx_ctx* c, const T* psi, int nband, int ld, const double* occ, double spn, double efac,
                         double* force, double* energy, bool use_k) {
@@ -2332,41 +2327,22 @@ int nonlocal_force_impl(lynx_ctx* c, const T* psi, int nband, int ld, const doub
     }
     LYNX_TRY(activate(c));
     const int na = c->nl.n_atom;
-    const int ncolp = ((nband + kNLColBlock - 1) / kNLColBlock) * kNLColBlock;
-    const size_t ab = sizeof(T) * (size_t)c->nl.total_proj * ncolp;
-    LYNX_TRY(c->alpha.ensure(ab));
-    LYNX_TRY(c->fbeta.ensure(ab));
-    LYNX_TRY(c->gradbuf[0].ensure(sizeof(T) * (size_t)c->Nd * nband));
+    LYNX_TRY(c->fpart.ensure(sphere_work_bytes(na, nband, false)));
     LYNX_TRY(c->fwork.ensure(sizeof(double) * ((size_t)nband + 4 * (size_t)na)));
-    const std::vector<double> ones(c->nl.total_proj, 1.0);
-    LYNX_TRY(c->fones.ensure(sizeof(double) * ones.size()));
-    LYNX_CUDA_TRY(cudaMemcpyAsync(c->fones.p, ones.data(), sizeof(double) * ones.size(), cudaMemcpyHostToDevice,
-                                  c->stream));
     double* docc = c->fwork.as<double>();
-    double* dforce = docc + nband;
-    double* dea = dforce + 3 * na;
+    double* dforce = docc + nband;  // [na][3], then the energies [na]
     LYNX_CUDA_TRY(cudaMemcpyAsync(docc, occ, sizeof(double) * nband, cudaMemcpyHostToDevice, c->stream));
-    NLDev raw = c->nl;  // projections without Gamma
-    raw.gamma = c->fones.as<double>();
     T phl[3], phr[3];
     ghost_phases<T>(c, use_k, phl, phr);
-    T* g = c->gradbuf[0].as<T>();
-    LYNX_TRY(launch_nl_gather<T>(raw, psi, l, nband, c->alpha.as<T>(), ncolp, c->dV, c->stream));
-    const double* D1[3] = {c->D1x.data(), c->D1y.data(), c->D1z.data()};
-    for (int d = 0; d < 3; ++d) {
-        LYNX_TRY(launch_grad_dir<T>(c->nx, c->ny, c->nz, c->nx, geom(c).R, D1[d], d, psi, l, g, c->Nd, nband, phl, phr,
-                                    c->stream));
-        LYNX_TRY(launch_nl_gather<T>(raw, g, c->Nd, nband, c->fbeta.as<T>(), ncolp, c->dV, c->stream));
-        LYNX_TRY(launch_nl_force_reduce<T>(c->nl, c->alpha.as<T>(), c->fbeta.as<T>(), ncolp, nband, docc, spn, efac, d,
-                                           dforce, dea, c->stream));
-    }
-    std::vector<double> ea(na);
-    LYNX_CUDA_TRY(cudaMemcpyAsync(force, dforce, sizeof(double) * 3 * na, cudaMemcpyDeviceToHost, c->stream));
-    LYNX_CUDA_TRY(cudaMemcpyAsync(ea.data(), dea, sizeof(double) * na, cudaMemcpyDeviceToHost, c->stream));
+    LYNX_TRY(launch_sphere_terms<T>(c->nl, force_geom(c), psi, l, nband, phl, phr, nullptr, docc, -spn, efac, c->dV,
+                                    false, c->fpart.as<double>(), dforce, dforce + 3 * na, c->stream));
+    std::vector<double> res(4 * (size_t)na);
+    LYNX_CUDA_TRY(cudaMemcpyAsync(res.data(), dforce, sizeof(double) * res.size(), cudaMemcpyDeviceToHost, c->stream));
     LYNX_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    std::copy(res.begin(), res.begin() + 3 * na, force);
     if (energy) {
         double e = 0.0;
-        for (int a = 0; a < na; ++a) e += ea[a];
+        for (int a = 0; a < na; ++a) e += res[3 * (size_t)na + a];
         *energy = e;
     }
     return LYNX_OK;
@@ -2389,9 +2365,8 @@ extern "C" int lynx_nonlocal_force_kpt(lynx_ctx* c, const double* psi_z, int nba
 //   stress_nl[ab] = -2 of sum_n g_n sum_j Gamma_j Re(conj(alpha_nj) beta^ab_nj) - delta_ab E_nl
 //   beta^ab = dV sum_img e^{-ik.R} chi (r - R_img)_b D_a psi,  E_nl = of sum g Gamma |alpha|^2
 // (src/physics/Stress.cpp:1041-1784; the GPU path's assembly src/physics/GPUForce.cu:471-680).
-// The relative positions enter through three copies of chi weighted by (r - R)_x, _y, _z, so
-// every beta is one gather of a gradient block; the sums over bands and atoms are finished on
-// the host in a fixed order.
+// The gradients are formed where they are used (forces.cu); the sums over bands run on the device, the
+// sum over atoms on the host, each in a fixed order.
 template <typename T>
 int stress_impl(lynx_ctx* c, const T* psi, int nband, int ld, const double* occ, double of, const double* img_pos,
                 double* stress_k, double* stress_nl, bool use_k) {
@@ -2401,109 +2376,36 @@ int stress_impl(lynx_ctx* c, const T* psi, int nband, int ld, const double* occ,
     LYNX_CHECK_ARG(l >= c->Nd, "ld < Nd");
     LYNX_CHECK_ARG(!c->has_nl || img_pos, "image positions are required when projectors are set");
     LYNX_TRY(activate(c));
-    const long long Nd = c->Nd;
-    const size_t gb = sizeof(T) * (size_t)Nd * nband;
-    LYNX_TRY(c->gradbuf[0].ensure(gb));
-    LYNX_TRY(c->gradbuf[1].ensure(gb));
-    LYNX_TRY(c->sbuf[0].ensure(gb));
-    T* G[3] = {c->gradbuf[0].as<T>(), c->gradbuf[1].as<T>(), c->sbuf[0].as<T>()};
+    const int na = c->has_nl ? c->nl.n_atom : 0;
+    const ForceGeom g = force_geom(c);
+    LYNX_TRY(c->fpart.ensure(std::max(kinetic_work_bytes(g, nband, ScalarOf<T>::cplx), sphere_work_bytes(na, nband, true))));
+    const size_t npos = c->has_nl ? 3 * (size_t)c->nl.n_img : 0;
+    LYNX_TRY(c->fwork.ensure(sizeof(double) * ((size_t)nband + npos + 7 * (size_t)na + 6)));
+    double* docc = c->fwork.as<double>();
+    double* dpos = docc + nband;
+    double* dres = dpos + npos;  // kinetic [6], then [na][6], then the energies [na]
+    LYNX_CUDA_TRY(cudaMemcpyAsync(docc, occ, sizeof(double) * nband, cudaMemcpyHostToDevice, c->stream));
+    if (npos)
+        LYNX_CUDA_TRY(cudaMemcpyAsync(dpos, img_pos, sizeof(double) * npos, cudaMemcpyHostToDevice, c->stream));
     T phl[3], phr[3];
     ghost_phases<T>(c, use_k, phl, phr);
-    const double* D1[3] = {c->D1x.data(), c->D1y.data(), c->D1z.data()};
-    for (int d = 0; d < 3; ++d)
-        LYNX_TRY(launch_grad_dir<T>(c->nx, c->ny, c->nz, c->nx, geom(c).R, D1[d], d, psi, l, G[d], Nd, nband, phl, phr,
-                                    c->stream));
-    if (!c->orth) {
-        // Cartesian gradients: D_cart = uvec^-1 D_lattice
-        const double* u = c->uvec;
-        const double det = u[0] * (u[4] * u[8] - u[5] * u[7]) - u[1] * (u[3] * u[8] - u[5] * u[6]) +
-                           u[2] * (u[3] * u[7] - u[4] * u[6]);
-        LYNX_CHECK_ARG(std::fabs(det) > 1e-14, "singular lattice");
-        const double ui[9] = {(u[4] * u[8] - u[5] * u[7]) / det, (u[2] * u[7] - u[1] * u[8]) / det,
-                              (u[1] * u[5] - u[2] * u[4]) / det, (u[5] * u[6] - u[3] * u[8]) / det,
-                              (u[0] * u[8] - u[2] * u[6]) / det, (u[2] * u[3] - u[0] * u[5]) / det,
-                              (u[3] * u[7] - u[4] * u[6]) / det, (u[1] * u[6] - u[0] * u[7]) / det,
-                              (u[0] * u[4] - u[1] * u[3]) / det};
-        LYNX_TRY(launch_cart_mix<T>(G[0], G[1], G[2], Nd * nband, ui, c->stream));
-    }
-    const int na = c->has_nl ? c->nl.n_atom : 0;
-    LYNX_TRY(c->fwork.ensure(sizeof(double) * (7 * (size_t)nband + 18 * (size_t)na + (size_t)na + 8)));
-    double* ddot = c->fwork.as<double>();  // [6][nband]
-    double* docc = ddot + 6 * nband;
-    double* dres = docc + nband;           // [6][na][3]
-    double* dea = dres + 18 * na;
-    LYNX_TRY(launch_dot6<T>(G[0], G[1], G[2], Nd, Nd, nband, ddot, c->stream));
-    std::vector<double> dots(6 * (size_t)nband);
-    LYNX_CUDA_TRY(cudaMemcpyAsync(dots.data(), ddot, sizeof(double) * dots.size(), cudaMemcpyDeviceToHost, c->stream));
-    LYNX_CUDA_TRY(cudaStreamSynchronize(c->stream));
-    for (int v = 0; v < 6; ++v) {
-        double sum = 0.0;
-        for (int n = 0; n < nband; ++n) sum += occ[n] * dots[(size_t)v * nband + n];
-        stress_k[v] = -of * c->dV * sum;
-        stress_nl[v] = 0.0;
-    }
-    if (!c->has_nl) return LYNX_OK;
-    // chi weighted by the Cartesian position relative to the image centre, per direction
-    const long long totchi = (long long)c->h_chi.size();
-    std::vector<double> wt[3];
-    for (auto& w : wt) w.assign(totchi, 0.0);
-    for (size_t im = 0; im < c->h_img_ndc.size(); ++im) {
-        const int ndc = c->h_img_ndc[im];
-        const int np = c->h_atom_nproj[c->h_img_atom[im]];
-        const long long go = c->h_img_goff[im], co = c->h_img_choff[im];
-        for (int ig = 0; ig < ndc; ++ig) {
-            const int gp = c->h_gpos[go + ig];
-            const int li = gp % c->nx, lj = (gp / c->nx) % c->ny, lk = gp / (c->nx * c->ny);
-            double r[3] = {li * c->dx - img_pos[3 * im], lj * c->dy - img_pos[3 * im + 1],
-                           lk * c->dz - img_pos[3 * im + 2]};
-            if (!c->orth) {
-                const double* u = c->uvec;  // cart_j = sum_i nc_i uvec(i, j)
-                const double a = r[0], b = r[1], e = r[2];
-                for (int j = 0; j < 3; ++j) r[j] = a * u[j] + b * u[3 + j] + e * u[6 + j];
-            }
-            for (int jp = 0; jp < np; ++jp) {
-                const long long k = co + (long long)jp * ndc + ig;
-                for (int b = 0; b < 3; ++b) wt[b][k] = c->h_chi[k] * r[b];
-            }
-        }
-    }
-    for (int b = 0; b < 3; ++b) {
-        LYNX_TRY(c->sbuf[1 + b].ensure(sizeof(double) * std::max<long long>(totchi, 2)));
-        LYNX_CUDA_TRY(cudaMemcpyAsync(c->sbuf[1 + b].p, wt[b].data(), sizeof(double) * totchi, cudaMemcpyHostToDevice,
-                                      c->stream));
-    }
-    const int ncolp = ((nband + kNLColBlock - 1) / kNLColBlock) * kNLColBlock;
-    const size_t ab = sizeof(T) * (size_t)c->nl.total_proj * ncolp;
-    LYNX_TRY(c->alpha.ensure(ab));
-    LYNX_TRY(c->fbeta.ensure(ab));
-    const std::vector<double> ones(c->nl.total_proj, 1.0);
-    LYNX_TRY(c->fones.ensure(sizeof(double) * std::max<size_t>(ones.size(), 1)));
-    LYNX_CUDA_TRY(cudaMemcpyAsync(c->fones.p, ones.data(), sizeof(double) * ones.size(), cudaMemcpyHostToDevice,
-                                  c->stream));
-    LYNX_CUDA_TRY(cudaMemcpyAsync(docc, occ, sizeof(double) * nband, cudaMemcpyHostToDevice, c->stream));
-    NLDev raw = c->nl;  // projections without Gamma
-    raw.gamma = c->fones.as<double>();
-    LYNX_TRY(launch_nl_gather<T>(raw, psi, l, nband, c->alpha.as<T>(), ncolp, c->dV, c->stream));
-    static const int va[6] = {0, 0, 0, 1, 1, 2}, vb[6] = {0, 1, 2, 1, 2, 2};
-    for (int v = 0; v < 6; ++v) {
-        NLDev w = raw;
-        w.chi64 = c->sbuf[1 + vb[v]].as<double>();
-        LYNX_TRY(launch_nl_gather<T>(w, G[va[v]], Nd, nband, c->fbeta.as<T>(), ncolp, c->dV, c->stream));
-        // per atom: -2 of sum_n g_n sum_j Gamma Re(conj(alpha) beta); slot v * 3 * na + a * 3 + (v ? 1 : 0);
-        // the energy shares with the first pair
-        LYNX_TRY(launch_nl_force_reduce<T>(c->nl, c->alpha.as<T>(), c->fbeta.as<T>(), ncolp, nband, docc, 2.0 * of, of,
-                                           v ? 1 : 0, dres + (size_t)v * 3 * na, dea, c->stream));
-    }
-    std::vector<double> res(18 * (size_t)na), ea(na);
+    bool phased = ScalarOf<T>::cplx;
+    for (int d = 0; d < 3; ++d) phased |= c->bc[d] != LYNX_BC_PERIODIC;
+    LYNX_TRY(launch_kinetic<T>(g, psi, l, nband, phl, phr, phased, docc, -of * c->dV, c->fpart.as<double>(), dres,
+                               c->stream));
+    if (na)
+        LYNX_TRY(launch_sphere_terms<T>(c->nl, g, psi, l, nband, phl, phr, dpos, docc, -2.0 * of, of, c->dV, true,
+                                        c->fpart.as<double>(), dres + 6, dres + 6 + 6 * na, c->stream));
+    std::vector<double> res(6 + 7 * (size_t)na);
     LYNX_CUDA_TRY(cudaMemcpyAsync(res.data(), dres, sizeof(double) * res.size(), cudaMemcpyDeviceToHost, c->stream));
-    LYNX_CUDA_TRY(cudaMemcpyAsync(ea.data(), dea, sizeof(double) * na, cudaMemcpyDeviceToHost, c->stream));
     LYNX_CUDA_TRY(cudaStreamSynchronize(c->stream));
     double enl = 0.0;
-    for (int a = 0; a < na; ++a) enl += ea[a];
+    for (int a = 0; a < na; ++a) enl += res[6 + 6 * (size_t)na + a];
     for (int v = 0; v < 6; ++v) {
+        stress_k[v] = res[v];
         double sum = 0.0;
-        for (int a = 0; a < na; ++a) sum += res[(size_t)v * 3 * na + (size_t)a * 3 + (v ? 1 : 0)];
-        stress_nl[v] = sum - ((v == 0 || v == 3 || v == 5) ? enl : 0.0);
+        for (int a = 0; a < na; ++a) sum += res[6 + (size_t)a * 6 + v];
+        stress_nl[v] = c->has_nl ? sum - ((v == 0 || v == 3 || v == 5) ? enl : 0.0) : 0.0;
     }
     return LYNX_OK;
 }
