@@ -43,13 +43,6 @@ int launch_direct_step(const StencilGeom& g, int nxp, const T* x, long long ldx,
                        long long ldout, const S* V, int ncol, double a, double b, double d, const T* phl,
                        const T* phr, const NonOrthGeom* ng, T* gy, T* gz, long long ldg, cudaStream_t st);
 
-// out = a*(-0.5*Lap x + V.*x) + b*x + d*xold over ncol columns (xold may be null when d == 0).
-// phl/phr: per-direction ghost multipliers (3 values of T each).
-template <typename T, typename S>
-int launch_cheb_step(const StencilGeom& g, const T* x, long long ldx, const T* xold, long long ldo, T* out,
-                     long long ldout, const S* V, int ncol, double a, double b, double d, const T* phl,
-                     const T* phr, cudaStream_t st);
-
 // Centre coefficient of a Chebyshev step, -0.5 a (D2x[0] + D2y[0] + D2z[0]) + b, for neighbour
 // coefficients c[p] = -0.5 a D2[p] stored in precision S, returned as a (hi, lo) pair in S.
 // FP32 (S = float): the centre is moved by the neighbours' rounding, -2 sum (c32 - c64), so the
@@ -95,8 +88,9 @@ int launch_cheb_pipe(const StencilGeom& g, int nxp, const T* x, long long ldx, c
                      int* err, cudaStream_t st, int shape = 0, const struct PipeNLHost* nlh = nullptr);
 // Number of launch shapes for FD half-width R: compiled shapes x two y-band splits (shape
 // indices 0 .. count-1; any shape gives bitwise the same result, they differ in speed only).
+// (odd nx: one).
 template <typename T>
-int pipe_shape_count(int R);
+int pipe_shape_count(int R, int nx);
 
 // Rayleigh-Ritz Gram products Ms = dV Y^T Y (upper triangle), Hs = dV Y^T HY of FP32 blocks
 // (rows x n, column stride ld) on the tensor cores: exact int8-slice products, FP64 result,

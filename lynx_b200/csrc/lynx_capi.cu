@@ -550,9 +550,15 @@ template <> struct Real<float2> { using type = float; };
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// The pipelined stencil pairs adjacent x points for real data, so it needs an even nx;
-// other grids keep unpadded rows and run the register-window kernel.
-template <typename T> bool pipe_capable(int nx) { return ScalarOf<T>::cplx || nx % 2 == 0; }
+// Grids whose blocks are kept in padded rows for the pipelined stencil: it pairs adjacent x points, and
+// takes an odd nx in periodic cells at FD order 12 (rows longer than kOddMaxNx may not fit its stages).
+// Other grids keep unpadded rows.  Complex blocks run the direct kernel, which takes any rows.
+constexpr int kOddMaxNx = 255;
+template <typename T> bool pipe_capable(const lynx_ctx* c) {
+    if (ScalarOf<T>::cplx || c->nx % 2 == 0) return true;
+    return c->R == 6 && c->nx <= kOddMaxNx && c->bc[0] == LYNX_BC_PERIODIC && c->bc[1] == LYNX_BC_PERIODIC &&
+           c->bc[2] == LYNX_BC_PERIODIC;
+}
 
 // Grows a work buffer; new storage is zeroed so that the padding elements of padded
 // row layouts read as zero.
@@ -709,7 +715,7 @@ int check_errflag(lynx_ctx* c) {
 
 // One fused step: out = a*(H_loc x) + b*x + d*xold, plus the nonlocal part a*Vnl x.
 // Blocks use rows of length nxp (nxp == nx: the caller's unpadded layout); V uses the same rows.
-// 16-byte aligned layouts run the pipelined kernel, others the register-window kernel.
+// 16-byte aligned layouts run the pipelined kernel, others the direct one.
 // Launch-shape autotuner of the pipelined stencil.  The first launch for a given (type, grid,
 // columns) times every compiled shape on the actual arguments (one untimed launch each, to load
 // the module, then one timed launch) and keeps the fastest for the context; every shape writes
@@ -720,7 +726,7 @@ int pipe_launch_tuned(lynx_ctx* c, int nxp, const T* x, long long ldx, const T* 
                       long long ldout, const S* V, int ncol, double a, double b, double d, const T* phl,
                       const T* phr, const PipeNLHost* nlh) {
     const StencilGeom g = geom(c);
-    const int nsh = pipe_shape_count<T>(g.R);
+    const int nsh = pipe_shape_count<T>(g.R, g.nx);
     const std::array<long long, 8> key = {(long long)sizeof(T), (long long)ScalarOf<T>::cplx, nxp, c->ny, c->nz,
                                           ncol, nlh != nullptr, xold != nullptr && d != 0.0};
     if (c->force_shape >= 0)
@@ -807,7 +813,7 @@ int cheb_step(lynx_ctx* c, int nxp, const T* x, long long ldx, const T* xold, lo
     using S = typename Real<T>::type;
     T phl[3], phr[3];
     ghost_phases<T>(c, use_k, phl, phr);
-    const bool pipe_ok = pipe_capable<T>(c->nx) && (nxp * sizeof(S)) % 16 == 0 && (ldx * sizeof(T)) % 16 == 0 &&
+    const bool pipe_ok = pipe_capable<T>(c) && (nxp * sizeof(S)) % 16 == 0 && (ldx * sizeof(T)) % 16 == 0 &&
                          (ldout * sizeof(T)) % 16 == 0 && (!xold || (ldo * sizeof(T)) % 16 == 0) && aligned16(x) &&
                          aligned16(out) && (!xold || aligned16(xold)) && aligned16(V);
     if (!pipe_ok && nxp != c->nx) {
@@ -824,7 +830,8 @@ int cheb_step(lynx_ctx* c, int nxp, const T* x, long long ldx, const T* xold, lo
                       c->nl.n_colors == 1 && geom(c).R == 6 && c->bc[0] == LYNX_BC_PERIODIC &&
                       c->bc[1] == LYNX_BC_PERIODIC && c->bc[2] == LYNX_BC_PERIODIC;
     const long long ldw = ((long long)c->nl.n_pts + 3) & ~3LL;  // compact column stride
-    const bool direct = ScalarOf<T>::cplx || (!fuse && c->force_shape < 0 && direct_step_pays<T>(c->Nd, ncol));
+    const bool direct =
+        ScalarOf<T>::cplx || !pipe_ok || (!fuse && c->force_shape < 0 && direct_step_pays<T>(c->Nd, ncol));
     const NLDev* nl = nullptr;
     if (c->has_nl) LYNX_TRY(nl_for(c, nxp, &nl));
     if (c->has_nl && !few) {
@@ -856,7 +863,7 @@ int cheb_step(lynx_ctx* c, int nxp, const T* x, long long ldx, const T* xold, lo
         if (c->time_stencil) LYNX_TRY(stencil_time_add(c));
     }
     if constexpr (!ScalarOf<T>::cplx) {
-        if (!direct && pipe_ok) {
+        if (!direct) {
             if (!c->errflag.p) LYNX_TRY(ensure_zeroed(c, c->errflag, sizeof(int)));
             if (fuse) {
                 const lynx_ctx::NLMap* nm = nullptr;
@@ -876,9 +883,6 @@ int cheb_step(lynx_ctx* c, int nxp, const T* x, long long ldx, const T* xold, lo
             LYNX_TRY(pipe_launch_tuned<T, S>(c, nxp, x, ldx, xold, ldo, out, ldout, V, ncol, a, b, d, phl, phr,
                                              nullptr));
             if (c->time_stencil) LYNX_TRY(stencil_time_add(c));
-        } else if (!direct) {
-            LYNX_TRY(launch_cheb_step<T, S>(geom(c), x, ldx, xold, ldo, out, ldout, V, ncol, a, b, d, phl, phr,
-                                            c->stream));
         }
     }
     if (!c->orth)
@@ -955,7 +959,7 @@ template <typename T64>
 int run_filter64(lynx_ctx* c, const T64* X, long long ldX, const double* veff, int N, double lc, double emin,
                  double emax, int degree, bool use_k, bool want_hy, T64** Y, T64** HY, long long* ldb, int* nxp) {
     using S = typename Real<T64>::type;
-    *nxp = pipe_capable<T64>(c->nx) ? pipe_row_elems(c->nx, sizeof(S)) : c->nx;
+    *nxp = pipe_capable<T64>(c) ? pipe_row_elems(c->nx, sizeof(S)) : c->nx;
     *ldb = (long long)(*nxp) * c->ny * c->nz;
     const size_t blk = sizeof(T64) * (size_t)(*ldb) * N;
     const bool direct = (*nxp == c->nx) && (ldX * sizeof(T64)) % 16 == 0 && aligned16(X);
@@ -985,7 +989,7 @@ template <typename T32, typename T64>
 int run_filter32(lynx_ctx* c, const T64* X, long long ldX, const double* veff, int N, double lc, double emin,
                  double emax, int degree, bool use_k, bool want_hy, T32** Y, T32** HY, long long* ldb, int* nxp) {
     using S = typename Real<T32>::type;
-    *nxp = pipe_capable<T32>(c->nx) ? pipe_row_elems(c->nx, sizeof(S)) : c->nx;
+    *nxp = pipe_capable<T32>(c) ? pipe_row_elems(c->nx, sizeof(S)) : c->nx;
     *ldb = (long long)(*nxp) * c->ny * c->nz;
     const size_t blk = sizeof(T32) * (size_t)(*ldb) * N;
     const int tag = (int)(sizeof(T32) * 1000 + *nxp);
@@ -1382,14 +1386,14 @@ int solve_impl(lynx_ctx* c, T64* psi, double* eig, const double* veff, int N, in
             return LYNX_OK;
         }
         if constexpr (std::is_same<T32, float>::value) {
-            if (pipe_capable<float>(c->nx) && !c->no_tc_gram) {
+            if (pipe_capable<float>(c) && !c->no_tc_gram) {
                 LYNX_TRY(rayleigh_ritz_mixed_real(c, Y, HY, ldb, nxp, reinterpret_cast<double*>(psi), ldp, N, eig));
                 LYNX_TRY(check_errflag(c));
                 if (lc_out) *lc_out = eig[N - 1] + 0.1;
                 return LYNX_OK;
             }
         } else {
-            if (pipe_capable<float>(c->nx) && rot_supported(2 * N) && !c->no_tc_gram) {
+            if (pipe_capable<float>(c) && rot_supported(2 * N) && !c->no_tc_gram) {
                 LYNX_TRY(rayleigh_ritz_mixed_cplx(c, Y, HY, ldb, nxp, reinterpret_cast<double2*>(psi), ldp, N, eig));
                 LYNX_TRY(check_errflag(c));
                 if (lc_out) *lc_out = eig[N - 1] + 0.1;
@@ -2119,7 +2123,7 @@ int lynx_eigensolver_solve_host(lynx_ctx* c, double* psi, double* eig, const dou
     // Mixed precision, real, pipelined layout: copy psi in column blocks (host_block columns, the
     // remainder last) on a second stream; the filter starts on a block as soon as it has landed
     // (see run_filter32).
-    const bool pipelined = precision == LYNX_PREC_MIXED && pipe_capable<float>(c->nx) && nband >= 256;
+    const bool pipelined = precision == LYNX_PREC_MIXED && pipe_capable<float>(c) && nband >= 256;
     std::vector<cudaEvent_t> evs;
     if (pipelined) {
         if (!c->copy_stream) LYNX_CUDA_TRY(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
@@ -2169,7 +2173,7 @@ int lynx_time_filter_step(lynx_ctx* c, const double* veff, int ncol, int precisi
     LYNX_CHECK_ARG(precision == LYNX_PREC_FP64 || precision == LYNX_PREC_MIXED, "unknown precision");
     LYNX_TRY(activate(c));
     const size_t esz = precision == LYNX_PREC_FP64 ? sizeof(double) : sizeof(float);
-    const int nxp = (c->nx % 2 == 0) ? pipe_row_elems(c->nx, esz) : c->nx;
+    const int nxp = pipe_capable<float>(c) ? pipe_row_elems(c->nx, esz) : c->nx;
     const long long ldb = (long long)nxp * c->ny * c->nz;
     for (int i = 0; i < 3; ++i) LYNX_TRY(ensure_layout(c, c->wbuf[i], esz * (size_t)ldb * ncol, (int)(esz * 1000 + nxp)));
     const bool nl = c->has_nl;

@@ -189,7 +189,7 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // through column offsets wrapped once at start-up, and PHASED instantiations (Bloch phases,
 // Dirichlet zeros) multiply wrapped neighbours in registers.  Per stage two mbarriers:
 // full (copies landed, tx-counted) and empty (every consumer warp done reading).
-template <typename T, int R, int RX, int RY, bool XOLD, int NS, bool PHASED, int MAXT, bool NLF>
+template <typename T, int R, int RX, int RY, bool XOLD, int NS, bool PHASED, int MAXT, bool NLF, bool ODD>
 __global__ void __launch_bounds__(MAXT, 1)
     cheb_pipe_kernel(const T* __restrict__ x, const T* __restrict__ xold, T* __restrict__ out,
                      const typename ScalarOf<T>::type* __restrict__ V, const PipeGeom G, const PipeCoef<T> C,
@@ -360,7 +360,9 @@ __global__ void __launch_bounds__(MAXT, 1)
     const T zero = vzero(T());
     // x-neighbour vectors: start columns wrapped into [0, nx) (nx is a multiple of RX, so a
     // vector never straddles the boundary); bit 2k / 2k+1 of xwrap: vector k wrapped left/right.
-    int xcol[NXV];
+    // ODD (nx odd, no phases): a wrapped vector would start on an odd element, so every element has an
+    // offset of its own (xcol: first elements, xcol1: second ones).
+    int xcol[NXV], xcol1[NXV];
     unsigned xwrap = 0;
 #pragma unroll
     for (int k = 0; k < NXV; ++k) {
@@ -373,6 +375,7 @@ __global__ void __launch_bounds__(MAXT, 1)
             xwrap |= 2u << (2 * k);
         }
         xcol[k] = c;
+        xcol1[k] = (ODD && c + 1 >= nx) ? c + 1 - nx : c + 1;
     }
     // y neighbours row R + yl +- p (staged rows); bit (r*2R + 2(p-1)) / +1: the row above / below
     // was copied across the y boundary (top rows wrap left, bottom rows wrap right).
@@ -445,9 +448,13 @@ __global__ void __launch_bounds__(MAXT, 1)
     const uint32_t rowbS = (uint32_t)(nxp * (int)sizeof(S));
     const uint32_t yoffb = (uint32_t)((yl[0] * nxp + xb) * (int)sizeof(T));
     const uint32_t soffb = (uint32_t)((yl[0] * nxp + xb) * (int)sizeof(S));
-    uint32_t xcolb[NXV];
+    uint32_t xcolb[NXV], xcolb1[NXV];
 #pragma unroll
-    for (int k = 0; k < NXV; ++k) xcolb[k] = (uint32_t)(xcol[k] * (int)sizeof(T));
+    for (int k = 0; k < NXV; ++k) {
+        xcolb[k] = (uint32_t)(xcol[k] * (int)sizeof(T));
+        xcolb1[k] = (uint32_t)(xcol1[k] * (int)sizeof(T));
+    }
+    const bool pad = ODD && xb + 1 >= nx;  // the thread's second point is row padding
     T* const othr = oc + (long long)z0 * G.plane + (long long)(y0 + yl[0]) * nxp + xb;
 
     auto window_entry = [&](int i, int z, VT* dst) -> bool {
@@ -509,7 +516,9 @@ __global__ void __launch_bounds__(MAXT, 1)
                 uint32_t ya = smem_u32(tile) + yoffb;  // row R + yl[0] + q for q = -R
 #pragma unroll
                 for (int q = -R; q < RY + R; ++q) {
-                    float2 v = lds<float2>(ya);
+                    float2 v;
+                    if (q >= 0 && q < RY && own[q]) v = w[J + R][q];  // an own row is in the window
+                    else v = lds<float2>(ya);
                     ya += rowb;
                     if (PHASED) {
                         if (ywrap_l & (1u << (q + R))) {
@@ -534,7 +543,10 @@ __global__ void __launch_bounds__(MAXT, 1)
                 float2 P[NXV];
 #pragma unroll
                 for (int k = 0; k < NXV; ++k) {
-                    float2 t = lds<float2>(ra + xcolb[k]);
+                    float2 t;
+                    if constexpr (ODD) t = make_float2(lds<float>(ra + xcolb[k]), lds<float>(ra + xcolb1[k]));
+                    else if (k == XOFF / RX) t = w[J + R][r];
+                    else t = lds<float2>(ra + xcolb[k]);
                     if (PHASED) {
                         if (xwrap & (1u << (2 * k))) {
                             t.x *= C.phl[0];
@@ -572,6 +584,7 @@ __global__ void __launch_bounds__(MAXT, 1)
                         if (m.y >= 0) xs[m.y] = acc[r].y;
                     }
                 }
+                if (ODD && pad) acc[r].y = 0.0f;
                 float* op = othr + (long long)(z - z0) * G.plane + r * nxp;
                 *reinterpret_cast<float2*>(op) = acc[r];
             }
@@ -614,7 +627,9 @@ __global__ void __launch_bounds__(MAXT, 1)
             uint32_t ya = smem_u32(tile) + yoffb;  // row R + yl[0] + q for q = -R
 #pragma unroll
             for (int q = -R; q < RY + R; ++q) {
-                VT v = lds<VT>(ya);
+                VT v;
+                if (q >= 0 && q < RY && own[q]) v = w[J + R][q];
+                else v = lds<VT>(ya);
                 ya += rowb;
                 T* ve = reinterpret_cast<T*>(&v);
                 if (PHASED) {
@@ -645,7 +660,16 @@ __global__ void __launch_bounds__(MAXT, 1)
                 T xv[NXV * RX];
 #pragma unroll
                 for (int k = 0; k < NXV; ++k) {
-                    VT t = lds<VT>(ra + xcolb[k]);
+                    VT t;
+                    if constexpr (ODD) {
+                        T* tp = reinterpret_cast<T*>(&t);
+                        tp[0] = lds<T>(ra + xcolb[k]);
+                        tp[1] = lds<T>(ra + xcolb1[k]);
+                    } else if (k == XOFF / RX) {
+                        t = w[J + R][r];
+                    } else {
+                        t = lds<VT>(ra + xcolb[k]);
+                    }
                     if (PHASED) {
                         T* tp = reinterpret_cast<T*>(&t);
                         if (xwrap & (1u << (2 * k))) {
@@ -701,7 +725,7 @@ __global__ void __launch_bounds__(MAXT, 1)
             VT o;
             T* opv = reinterpret_cast<T*>(&o);
 #pragma unroll
-            for (int u = 0; u < RX; ++u) opv[u] = acc[r][u];
+            for (int u = 0; u < RX; ++u) opv[u] = (ODD && pad && u > 0) ? zero : acc[r][u];
             *reinterpret_cast<VT*>(op) = o;
         }
         }

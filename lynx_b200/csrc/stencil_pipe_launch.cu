@@ -29,6 +29,10 @@ template <typename T> struct NumShapes { static constexpr int value = 1; };
 template <> struct NumShapes<float> { static constexpr int value = 4; };
 template <> struct NumShapes<double> { static constexpr int value = 4; };
 constexpr int kTunedR = 6;  // FD order 12
+// Odd nx (kTunedR, periodic cells): one shape per type, the one the autotuner keeps most often.
+template <typename T> struct OddShape;
+template <> struct OddShape<float> { static constexpr int value = 1; };
+template <> struct OddShape<double> { static constexpr int value = 2; };
 constexpr int kFewCtas = 2 * 148;  // below this many CTAs, bands and z chunks are made shorter
 constexpr int kMinChunk = 4;       // planes of the shortest z chunk
 
@@ -53,15 +57,15 @@ ShapeRT shape_rt(int si) {
     return shape_i<T, 0>();
 }
 
-template <typename T, int R, bool XOLD, bool PH, int SI, bool NLF = false>
+template <typename T, int R, bool XOLD, bool PH, int SI, bool NLF = false, bool ODD = false>
 void launch_pipe_ph(int ns, dim3 grid, int nthr, size_t smem, cudaStream_t st, const T* x, const T* xo, T* out,
                     const typename ScalarOf<T>::type* V, const PipeGeom& G, const PipeCoef<T>& C,
                     const PipeNL<T>& NL, int* err) {
     using P = PipeShapeAt<T, SI>;
     constexpr int RX = P::RX, RY = P::RY, MT = P::MAXT;
-    auto kern = ns >= 5 ? cheb_pipe_kernel<T, R, RX, RY, XOLD, 5, PH, MT, NLF>
-               : (ns == 4 ? cheb_pipe_kernel<T, R, RX, RY, XOLD, 4, PH, MT, NLF>
-                          : cheb_pipe_kernel<T, R, RX, RY, XOLD, 3, PH, MT, NLF>);
+    auto kern = ns >= 5 ? cheb_pipe_kernel<T, R, RX, RY, XOLD, 5, PH, MT, NLF, ODD>
+               : (ns == 4 ? cheb_pipe_kernel<T, R, RX, RY, XOLD, 4, PH, MT, NLF, ODD>
+                          : cheb_pipe_kernel<T, R, RX, RY, XOLD, 3, PH, MT, NLF, ODD>);
     smem_cap(kern, smem);
     kern<<<grid, nthr, smem, st>>>(x, xo, out, V, G, C, NL, err);
 }
@@ -69,14 +73,20 @@ void launch_pipe_ph(int ns, dim3 grid, int nthr, size_t smem, cudaStream_t st, c
 // Real data with periodic boundaries needs no phase on wrapped neighbours; complex data and
 // Dirichlet boundaries use the PHASED instantiation (default shape only).
 template <typename T, int R, bool XOLD>
-void launch_pipe(int si, int ns, bool phased, bool nlf, dim3 grid, int nthr, size_t smem, cudaStream_t st, const T* x,
+void launch_pipe(int si, int ns, bool phased, bool nlf, bool odd, dim3 grid, int nthr, size_t smem, cudaStream_t st, const T* x,
                  const T* xo, T* out, const typename ScalarOf<T>::type* V, const PipeGeom& G, const PipeCoef<T>& C,
                  const PipeNL<T>& NL, int* err) {
-    if (ScalarOf<T>::cplx || phased) {
+    if (phased) {
         launch_pipe_ph<T, R, XOLD, true, 0>(ns, grid, nthr, smem, st, x, xo, out, V, G, C, NL, err);
         return;
     }
     if constexpr (R == kTunedR && NumShapes<T>::value > 1) {
+        if (odd) {
+            constexpr int SI = OddShape<T>::value;
+            if (nlf) launch_pipe_ph<T, R, XOLD, false, SI, true, true>(ns, grid, nthr, smem, st, x, xo, out, V, G, C, NL, err);
+            else launch_pipe_ph<T, R, XOLD, false, SI, false, true>(ns, grid, nthr, smem, st, x, xo, out, V, G, C, NL, err);
+            return;
+        }
         if (nlf) {
             switch (si) {
                 case 1: launch_pipe_ph<T, R, XOLD, false, 1, true>(ns, grid, nthr, smem, st, x, xo, out, V, G, C, NL, err); return;
@@ -110,9 +120,9 @@ bool phases_trivial(const T* phl, const T* phr) {
 }  // namespace
 
 template <typename T>
-int pipe_shape_count(int R) {
+int pipe_shape_count(int R, int nx) {
     // shapes x band splits: index = shape + NumShapes * (extra y-bands, 0 or 1)
-    return (R == kTunedR && NumShapes<T>::value > 1) ? 2 * NumShapes<T>::value : 1;
+    return (R == kTunedR && NumShapes<T>::value > 1 && nx % 2 == 0) ? 2 * NumShapes<T>::value : 1;
 }
 
 template <typename T, typename S>
@@ -121,14 +131,19 @@ int launch_cheb_pipe(const StencilGeom& g, int nxp, const T* x, long long ldx, c
                      int* err, cudaStream_t st, int shape, const PipeNLHost* nlh) {
     static_assert(std::is_same<S, typename ScalarOf<T>::type>::value, "scalar type mismatch");
     const int R = g.R;
-    const bool phased = ScalarOf<T>::cplx || !phases_trivial(phl, phr);
+    const bool phased = !phases_trivial(phl, phr);
     const bool nlf = nlh != nullptr;
     if (nlf && (R != kTunedR || phased || NumShapes<T>::value == 1)) {
         set_error("fused nonlocal term needs real data, periodic cells and FD order 12");
         return LYNX_ERR_UNSUPPORTED;
     }
-    const int sidx = (shape > 0 && shape < pipe_shape_count<T>(R) && !phased) ? shape : 0;
-    const int si = sidx % NumShapes<T>::value;    // compiled launch shape
+    const bool odd = g.nx % 2 != 0;
+    if (odd && (R != kTunedR || phased)) {
+        set_error("the pipelined stencil takes an odd nx in periodic cells at FD order 12 only");
+        return LYNX_ERR_UNSUPPORTED;
+    }
+    const int sidx = (shape > 0 && shape < pipe_shape_count<T>(R, g.nx) && !phased) ? shape : 0;
+    const int si = odd ? OddShape<T>::value : sidx % NumShapes<T>::value;  // compiled launch shape
     const int extra_bands = sidx / NumShapes<T>::value;  // one more y-band: more, shorter CTAs
     const ShapeRT sh = shape_rt<T>(si);
     const int RX = sh.RX, RY = sh.RY, MT = sh.MAXT;
@@ -145,12 +160,8 @@ int launch_cheb_pipe(const StencilGeom& g, int nxp, const T* x, long long ldx, c
         set_error("pipelined stencil needs 16-byte aligned rows and columns");
         return LYNX_ERR_BAD_ARG;
     }
-    if (g.nx % RX != 0) {
-        set_error("pipelined stencil needs nx to be a multiple of %d", RX);
-        return LYNX_ERR_UNSUPPORTED;
-    }
     if (ncol <= 0) return LYNX_OK;
-    const int P2 = g.nx / RX;
+    const int P2 = (g.nx + RX - 1) / RX;
     if (P2 > MT - 32) {
         set_error("nx = %d too large for the pipelined stencil", g.nx);
         return LYNX_ERR_UNSUPPORTED;
@@ -244,8 +255,8 @@ int launch_cheb_pipe(const StencilGeom& g, int nxp, const T* x, long long ldx, c
     dim3 grid(nbands, ncol, nzch);
 #define LYNX_PIPE_CASE(RR)                                                                       \
     case RR:                                                                                     \
-        if (xo) launch_pipe<T, RR, true>(si, ns, phased, nlf, grid, nthr, smem, st, x, xold, out, V, G, C, NL, err); \
-        else launch_pipe<T, RR, false>(si, ns, phased, nlf, grid, nthr, smem, st, x, xold, out, V, G, C, NL, err);   \
+        if (xo) launch_pipe<T, RR, true>(si, ns, phased, nlf, odd, grid, nthr, smem, st, x, xold, out, V, G, C, NL, err); \
+        else launch_pipe<T, RR, false>(si, ns, phased, nlf, odd, grid, nthr, smem, st, x, xold, out, V, G, C, NL, err);   \
         break;
     switch (R) {
         LYNX_PIPE_CASE(1)
@@ -273,7 +284,7 @@ template int launch_cheb_pipe<double, double>(const StencilGeom&, int, const dou
 template int launch_cheb_pipe<float, float>(const StencilGeom&, int, const float*, long long, const float*,
                                             long long, float*, long long, const float*, int, double, double, double,
                                             const float*, const float*, int*, cudaStream_t, int, const PipeNLHost*);
-template int pipe_shape_count<double>(int);
-template int pipe_shape_count<float>(int);
+template int pipe_shape_count<double>(int, int);
+template int pipe_shape_count<float>(int, int);
 
 }  // namespace lynxb

@@ -1,0 +1,61 @@
+"""Odd nx in the pipelined stencil (padded rows, element-wise wrapped x neighbours) and in the
+tensor-core Rayleigh-Ritz step that its padded blocks allow, against the numpy oracle; rows that end
+one or two points past a thread block, with and without the fused nonlocal term."""
+import numpy as np
+import pytest
+
+from lynx_b200 import _lib
+from lynx_b200 import cell as C
+from lynx_b200 import pseudo as P
+from oracle import chefsi_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _system(synth_psp8, reps, shape):
+    from lynx_b200 import solver
+    cl, pos = C.diamond_si(reps, shape, displace=0.02, seed=9)
+    V = C.synthetic_veff_separable(cl, pos, noise=1e-3, seed=9)
+    tab = P.nonlocal_tables(cl, pos, P.read_psp8(synth_psp8))
+    ctx = solver.Context(cl)
+    ctx.set_nonlocal(tab)
+    t = dict(img_atom=tab.img_atom, img_ndc=tab.img_ndc, img_shift=tab.img_shift, gpos=tab.gpos, chi=tab.chi,
+             gamma=tab.gamma, nproj=int(tab.atom_nproj[0]))
+    return solver, ctx, V, O.Operator(cl.latvec, cl.shape, 12, True, t)
+
+
+# FP64: 3 steps of sums of 60 terms; FP32: the same at 2^-24 per operation (measured 1e-6 of the largest)
+@pytest.mark.parametrize("shape", [(49, 50, 52), (51, 48, 49), (53, 51, 50), (55, 49, 48)])
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-13), ("mixed", 1e-5)])
+@pytest.mark.parametrize("fuse", [1, 0])
+def test_filter(synth_psp8, shape, precision, tol, fuse):
+    solver, ctx, V, H = _system(synth_psp8, 2, shape)
+    ctx.set_option(_lib.OPT_FUSE_NONLOCAL, fuse)
+    x = C.random_orbitals(ctx.nd, 3, seed=2)
+    y = solver.EigenSolver(ctx, precision).chebyshev_filter(x, V, 25.0, -2.0, 70.0, degree=3)
+    want = O.chebyshev_filter(H, x, V, 25.0, -2.0, 70.0, 3)
+    assert np.abs(y - want).max() < tol * np.abs(want).max()
+    ctx.close()
+
+
+@pytest.mark.parametrize("n", [41, 130])
+def test_mixed_pass(synth_psp8, n):
+    """The tensor-core products of odd rows against FP64 library products of the same filtered block,
+    and the density accumulated in the rotation against the density of the orbitals."""
+    import torch
+    solver, ctx, V, _ = _system(synth_psp8, 1, (25, 26, 27))
+    es = solver.EigenSolver(ctx, "mixed")
+    x = np.ascontiguousarray(C.random_orbitals(ctx.nd, n, seed=3).T)
+    lo, hi = float(V.min()) - 1.0, ctx.max_eigval_half_lap + 8.0
+    out = []
+    for tc in (1, 0):
+        ctx.set_option(_lib.OPT_TC_RAYLEIGH_RITZ, tc)
+        psi = torch.from_numpy(x).cuda()
+        _, eig, rho, ef = es.solve_density(psi, V, 0.5 * (lo + hi), lo, hi, 8, nelectron=32.0)
+        w = solver.electron_density(ctx, psi, solver.occupations(eig, ef, 1000.0))
+        assert float((rho - w).abs().max()) < 1e-12 * float(w.abs().max())
+        s = (psi @ psi.T).cpu().numpy() * ctx.dV
+        assert np.abs(s - np.eye(n)).max() < 1e-5
+        out.append(eig)
+    assert np.abs(out[0] - out[1]).max() < 2e-7 * np.abs(out[1]).max()
+    ctx.close()
