@@ -168,13 +168,15 @@ struct DotList {
     const double* u[kMaxDots];
     const double* v[kMaxDots];
 };
-int launch_grad3(const double* x, const GradGeom& g, double* dx, double* dy, double* dz, cudaStream_t st);
-int launch_div_sub(double* v, const GradGeom& g, const double* fx, const double* fy, const double* fz,
-                   cudaStream_t st);
 int launch_rho_xc(const double* rho, const double* core, double* out, long long nd, cudaStream_t st);
-// GGA-PBE per point; on return gx, gy, gz hold the GGA flux v2xc lapc_T grad(rho).
-int launch_pbe(const double* rho, long long nd, const XcMetric& m, double* gx, double* gy, double* gz, double* vxc,
-               double* exc, double* v2xc, cudaStream_t st);
+// Gradient of rho, GGA-PBE per point and the GGA flux v2xc lapc_T grad(rho) in fx, fy, fz; with rhs also
+// 4 pi (rho0 + rho_b) (rho_b may be null).
+int launch_grad_pbe(const double* rho, const GradGeom& g, const XcMetric& m, double* fx, double* fy, double* fz,
+                    double* vxc, double* exc, double* v2xc, const double* rho0, const double* rho_b, double* rhs,
+                    cudaStream_t st);
+// v -= div f; with phi also veff = v + phi.
+int launch_div_sub(double* v, const GradGeom& g, const double* fx, const double* fy, const double* fz,
+                   const double* phi, double* veff, cudaStream_t st);
 int launch_aar_pre(const double* r, const double* x, double* x_old, double* f, double* f_old, double* X, double* F,
                    double w, long long n, cudaStream_t st);
 int launch_aar_update(double* x, const double* x_old, const double* f, const double* X, const double* F,

@@ -2841,30 +2841,36 @@ int field_sum(lynx_ctx* c, const double* x, double* sum) {
 
 }  // namespace
 
+// Gradient, functional and flux of the exchange-correlation part (asynchronous); *f: the three flux
+// fields that launch_div_sub takes.  With rhs also the Poisson right-hand side.
+static int xc_terms(lynx_ctx* c, const double* rho, const double* rho_core, double* vxc, double* exc,
+                    double* dxcdgrho, const double* rho_b, double* rhs, double** f) {
+    const long long N = c->Nd;
+    // scratch: 3 flux fields, the core-corrected density, the Poisson right-hand side
+    LYNX_TRY(c->xcwork.ensure(sizeof(double) * (size_t)N * 5));
+    *f = c->xcwork.as<double>();
+    const double* rx = rho;
+    if (rho_core) {
+        double* t = *f + 3 * N;
+        LYNX_TRY(launch_rho_xc(rho, rho_core, t, N, c->stream));
+        rx = t;
+    }
+    XcMetric mt{};
+    mt.orth = c->orth ? 1 : 0;
+    for (int i = 0; i < 9; ++i) mt.L[i] = c->lapcT[i];
+    return launch_grad_pbe(rx, grad_geom(c), mt, *f, *f + N, *f + 2 * N, vxc, exc, dxcdgrho, rho, rho_b, rhs,
+                           c->stream);
+}
+
 extern "C" int lynx_xc_gga_pbe(lynx_ctx* c, const double* rho, const double* rho_core, double* vxc, double* exc,
                                double* dxcdgrho) {
     LYNX_CHECK_ARG(c && rho && vxc && exc, "null pointer");
     LYNX_CHECK_ARG(c->nx > c->R && c->ny > c->R && c->nz > c->R, "grid smaller than the FD half-width");
     LYNX_TRY(activate(c));
     const long long N = c->Nd;
-    // scratch: 3 gradient / flux fields and the core-corrected density
-    LYNX_TRY(c->xcwork.ensure(sizeof(double) * (size_t)N * 4));
-    double* gx = c->xcwork.as<double>();
-    double* gy = gx + N;
-    double* gz = gy + N;
-    const double* rx = rho;
-    if (rho_core) {
-        double* t = gz + N;
-        LYNX_TRY(launch_rho_xc(rho, rho_core, t, N, c->stream));
-        rx = t;
-    }
-    const GradGeom g = grad_geom(c);
-    LYNX_TRY(launch_grad3(rx, g, gx, gy, gz, c->stream));
-    XcMetric mt{};
-    mt.orth = c->orth ? 1 : 0;
-    for (int i = 0; i < 9; ++i) mt.L[i] = c->lapcT[i];
-    LYNX_TRY(launch_pbe(rx, N, mt, gx, gy, gz, vxc, exc, dxcdgrho, c->stream));
-    LYNX_TRY(launch_div_sub(vxc, g, gx, gy, gz, c->stream));
+    double* f = nullptr;
+    LYNX_TRY(xc_terms(c, rho, rho_core, vxc, exc, dxcdgrho, nullptr, nullptr, &f));
+    LYNX_TRY(launch_div_sub(vxc, grad_geom(c), f, f + N, f + 2 * N, nullptr, nullptr, c->stream));
     LYNX_CUDA_TRY(cudaStreamSynchronize(c->stream));
     return LYNX_OK;
 }
@@ -2886,6 +2892,21 @@ extern "C" int lynx_effective_potential(lynx_ctx* c, const double* rho, const do
     LYNX_CHECK_ARG(poisson_tol > 0.0, "poisson_tol must be positive");
     LYNX_TRY(activate(c));
     const long long N = c->Nd;
+    const bool periodic = c->bc[0] == LYNX_BC_PERIODIC && c->bc[1] == LYNX_BC_PERIODIC && c->bc[2] == LYNX_BC_PERIODIC;
+    if (c->poisson_direct && periodic) {
+        // No host step in between: the mean of the right-hand side and of phi is the Fourier mode that the
+        // inverse symbol sets to zero, and V_eff is added up where the divergence is.
+        LYNX_CHECK_ARG(c->nx > c->R && c->ny > c->R && c->nz > c->R, "grid smaller than the FD half-width");
+        LYNX_TRY(c->xcwork.ensure(sizeof(double) * (size_t)N * 5));
+        double* rhs = c->xcwork.as<double>() + 4 * N;
+        double* f = nullptr;
+        LYNX_TRY(xc_terms(c, rho, rho_core, vxc, exc, nullptr, rho_b, rhs, &f));
+        LYNX_TRY(poisson_direct(c, rhs, phi));
+        LYNX_TRY(launch_div_sub(vxc, grad_geom(c), f, f + N, f + 2 * N, phi, veff, c->stream));
+        LYNX_CUDA_TRY(cudaStreamSynchronize(c->stream));
+        if (poisson_iters) *poisson_iters = 0;
+        return LYNX_OK;
+    }
     // 1. exchange-correlation
     LYNX_TRY(lynx_xc_gga_pbe(c, rho, rho_core, vxc, exc, nullptr));
     // 2. Poisson: rhs = 4 pi rho + 4 pi rho_b with its mean removed;
@@ -2895,13 +2916,7 @@ extern "C" int lynx_effective_potential(lynx_ctx* c, const double* rho, const do
     double sum = 0.0;
     LYNX_TRY(field_sum(c, veff, &sum));
     LYNX_TRY(launch_add_shift(veff, nullptr, sum / (double)N, 1.0, veff, N, c->stream));
-    const bool periodic = c->bc[0] == LYNX_BC_PERIODIC && c->bc[1] == LYNX_BC_PERIODIC && c->bc[2] == LYNX_BC_PERIODIC;
-    if (c->poisson_direct && periodic) {
-        LYNX_TRY(poisson_direct(c, veff, phi));
-        if (poisson_iters) *poisson_iters = 0;
-    } else {
-        LYNX_TRY(poisson_aar(c, veff, phi, poisson_tol, 3000, poisson_iters));
-    }
+    LYNX_TRY(poisson_aar(c, veff, phi, poisson_tol, 3000, poisson_iters));
     // phi shifted to zero mean (EffectivePotential.cpp:64-70)
     LYNX_TRY(field_sum(c, phi, &sum));
     LYNX_TRY(launch_add_shift(phi, nullptr, sum / (double)N, 1.0, phi, N, c->stream));
