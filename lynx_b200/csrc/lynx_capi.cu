@@ -612,14 +612,14 @@ int repack(lynx_ctx* c, Dst* dst, int dnxp, long long dld, const Src* src, int s
     return LYNX_OK;
 }
 
-// Uploads a host table into a buffer of its own, complete on return.  On the context's stream and
-// waited for: a plain cudaMemcpy from pageable memory may return while its copy is still under way
-// on the legacy stream, which kernels on a non-blocking stream do not wait for.
+// Uploads a host table into a buffer of its own, on the context's stream: a plain cudaMemcpy from
+// pageable memory may return while its copy is still under way on the legacy stream, which kernels on a
+// non-blocking stream do not wait for.  (The source may go: pageable memory is staged before the call
+// returns.)
 int upload_table(lynx_ctx* c, DevBuf& b, const void* src, size_t bytes) {
     LYNX_TRY(b.ensure(std::max<size_t>(bytes, 16)));
     if (!bytes) return LYNX_OK;
     LYNX_CUDA_TRY(cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, c->stream));
-    LYNX_CUDA_TRY(cudaStreamSynchronize(c->stream));
     return LYNX_OK;
 }
 
@@ -652,6 +652,7 @@ int nl_for(lynx_ctx* c, int nxp, const NLDev** out) {
     c->nl_layout_bufs.emplace_back();
     DevBuf& b2 = c->nl_layout_bufs.back();
     LYNX_TRY(upload_table(c, b2, pg.data(), pg.size() * 4));
+    LYNX_CUDA_TRY(cudaStreamSynchronize(c->stream));  // the context may change streams
     d.pt_grid = b2.as<int>();
     c->nl_layouts[nxp] = d;
     *out = &c->nl_layouts[nxp];
@@ -682,6 +683,7 @@ int nl_map_for(lynx_ctx* c, int nxp, const lynx_ctx::NLMap** out) {
     for (long long r = 0; r < rows; ++r) m.rowstart_h[r + 1] += m.rowstart_h[r];
     LYNX_TRY(upload_table(c, m.ptmap, pm.data(), pm.size() * sizeof(int)));
     LYNX_TRY(upload_table(c, m.rowstart, m.rowstart_h.data(), m.rowstart_h.size() * sizeof(int)));
+    LYNX_CUDA_TRY(cudaStreamSynchronize(c->stream));
     *out = &m;
     return LYNX_OK;
 }
@@ -1143,7 +1145,9 @@ int rayleigh_ritz_real(lynx_ctx* c, const double* Y, long long ldY, const double
                        double* psi, long long ldp, int N, double* eig_host) {
     LYNX_TRY(rr_alloc_small(c, N, sizeof(double)));
     const double dV = c->dV, zero = 0.0;
-    CUBLAS_TRY(cublasDsyrk(c->cublas, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_T, N, c->Nd, &dV, Y, ldY, &zero,
+    // The overlap as a full product: the library splits the long K of a GEMM over the SMs, but not that of
+    // a rank-k update (Si64, 160 states: 0.43 ms against 2.8).
+    CUBLAS_TRY(cublasDgemm(c->cublas, CUBLAS_OP_T, CUBLAS_OP_N, N, N, c->Nd, &dV, Y, ldY, Y, ldY, &zero,
                            c->Ms.as<double>(), N));
     CUBLAS_TRY(cublasDgemm(c->cublas, CUBLAS_OP_T, CUBLAS_OP_N, N, N, c->Nd, &dV, Y, ldY, HY, ldH, &zero,
                            c->Hs.as<double>(), N));

@@ -26,6 +26,30 @@ cudaError_t smem_cap(K* kern, size_t bytes) {
     return raise_smem_cap(reinterpret_cast<const void*>(kern), bytes);
 }
 
+// Programmatic dependent launch for the chains of short kernels of the filter: the next kernel's blocks
+// may be set up while this one still runs, and wait in pdl_wait() for all of its results.  Every kernel
+// launched this way calls pdl_wait() before it touches memory that an earlier kernel may read or write.
+#ifdef __CUDACC__
+__device__ __forceinline__ void pdl_wait() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... P, typename... A>
+cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+#endif
+
 }  // namespace lynxb
 
 #define LYNX_CUDA_TRY(...)                                                                      \

@@ -16,6 +16,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include "kernels.h"
+#include "lynx_common.cuh"
 #include "stencil.cuh"
 
 namespace lynxb {
@@ -94,14 +95,16 @@ constexpr int fold_slots() {  // values left per lane after R rounds
 // columns; its eight warps take the atom's steps of 32 points in turn.  A lane loads its point's NP
 // projector values and NC values of x (both coalesced along the points) and keeps the NC x NP sums in
 // registers, so there is no staging, no barrier and no chain between steps: many loads are in flight
-// even when an atom has few points and few columns.  The sums over the lanes are folded, and the
-// warps are added in shared memory in a fixed order.  Complex data: the sums of one image, times the
-// image's phase, are added up per image.
+// even when an atom has few points and few columns.  (The images' table entries, a chain of dependent
+// loads, are read once for all of them.)  The sums over the lanes are folded, and the warps are added in
+// shared memory in a fixed order.  Complex data: x is multiplied by the image's Bloch phase (FP64) as
+// it is read.
 //
 // APPLY: the same CTA then adds the projectors' term, out[g] += scale * sum_j chi[j, g] alpha[j], at
 // its atom's points (j in order from zero, the order of the scatter kernels, so bitwise their
 // result).  Only when no grid point lies in two spheres: then every point has one writer.  alpha
 // does not leave the CTA.
+constexpr int kAtomImgs = 32;
 template <typename T, int NP, int NC, bool APPLY>
 __global__ void __launch_bounds__(256)
     nl_atom_kernel(const T* __restrict__ x, long long ld, int ncol, int ncolp, NLView tab, T* __restrict__ alpha,
@@ -118,25 +121,40 @@ __global__ void __launch_bounds__(256)
     const int i0 = tab.atom_img_ptr[a], i1 = tab.atom_img_ptr[a + 1];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int n0 = blockIdx.x * NC;
+    // table entries of up to kAtomImgs images at a time
+    __shared__ int im_ndc[kAtomImgs];
+    __shared__ const int* im_gp[kAtomImgs];
+    __shared__ const S* im_ch[kAtomImgs];
+    __shared__ double2 im_ph[kAtomImgs];
+    auto images = [&](int ic) -> int {  // entries ic .. of the atom's list; all threads
+        const int n = min(kAtomImgs, i1 - ic);
+        __syncthreads();
+        if ((int)threadIdx.x < n) {
+            const int im = tab.atom_img_list[ic + threadIdx.x];
+            im_ndc[threadIdx.x] = tab.img_ndc[im];
+            im_gp[threadIdx.x] = tab.gpos + tab.img_goff[im];
+            im_ch[threadIdx.x] = chi + tab.img_chi_off[im];
+            if (ScalarOf<T>::cplx) im_ph[threadIdx.x] = make_double2(tab.img_phase[2 * im], tab.img_phase[2 * im + 1]);
+        }
+        __syncthreads();
+        return n;
+    };
+    if (i1 - i0 <= kAtomImgs) images(i0);  // the tables are nobody's results
+    pdl_wait();
     T acc[M];  // [projector][column]
 #pragma unroll
     for (int q = 0; q < M; ++q) acc[q] = vzero(T());
-    if (n0 < ncol) {
-        const T* xc[NC];
+    const T* xc[NC];
 #pragma unroll
-        for (int c = 0; c < NC; ++c) xc[c] = x + (long long)min(n0 + c, ncol - 1) * ld;
-        int q0 = 0;  // steps of the images before this one
-        for (int ii = i0; ii < i1; ++ii) {
-            const int im = tab.atom_img_list[ii];
-            const int ndc = tab.img_ndc[im];
+    for (int c = 0; c < NC; ++c) xc[c] = x + (long long)min(n0 + c, ncol - 1) * ld;
+    int q0 = 0;  // steps of the images before this one
+    for (int ic = i0; ic < i1 && n0 < ncol; ic += kAtomImgs) {
+        const int ni = i1 - i0 <= kAtomImgs ? i1 - i0 : images(ic);
+        for (int ii = 0; ii < ni; ++ii) {
+            const int ndc = im_ndc[ii];
             const int nst = (ndc + 31) >> 5;
-            const int* gp = tab.gpos + tab.img_goff[im];
-            const S* ch = chi + tab.img_chi_off[im];
-            T sum[ScalarOf<T>::cplx ? M : 1];
-            if constexpr (ScalarOf<T>::cplx) {
-#pragma unroll
-                for (int q = 0; q < M; ++q) sum[q] = vzero(T());
-            }
+            const int* gp = im_gp[ii];
+            const S* ch = im_ch[ii];
 #pragma unroll 2
             for (int s = (w - q0) & 7; s < nst; s += 8) {
                 const int g = 32 * s + lane;
@@ -147,27 +165,20 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
                     xv[c] = xc[c][o];
+                    if constexpr (ScalarOf<T>::cplx) xv[c] = acc_phase(xv[c], im_ph[ii].x, im_ph[ii].y);
                     if (!ok) xv[c] = vzero(T());
                 }
 #pragma unroll
                 for (int j = 0; j < NP; ++j) {
                     const S cv = ch[(long long)min(j, np - 1) * ndc + gc];
 #pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        if constexpr (ScalarOf<T>::cplx) sum[j * NC + c] = fmac(sum[j * NC + c], cv, xv[c]);
-                        else acc[j * NC + c] = fmac(acc[j * NC + c], cv, xv[c]);
-                    }
+                    for (int c = 0; c < NC; ++c) acc[j * NC + c] = fmac(acc[j * NC + c], cv, xv[c]);
                 }
             }
             q0 += nst;
-            if constexpr (ScalarOf<T>::cplx) {
-                const double re = tab.img_phase[2 * im], ph = tab.img_phase[2 * im + 1];
-#pragma unroll
-                for (int q = 0; q < M; ++q) acc[q] = vadd(acc[q], acc_phase(sum[q], re, ph));
-            }
         }
-        warp_fold<M, 16>(acc, lane);
     }
+    if (n0 < ncol) warp_fold<M, 16>(acc, lane);
 #pragma unroll
     for (int i = 0; i < fold_slots<M, 5>(); ++i) {
         const int q = fold_index<M, 16>(i, lane);
@@ -189,44 +200,47 @@ __global__ void __launch_bounds__(256)
         else if (n < ncolp) alpha[(long long)(poff + j) * ncolp + n] = n < ncol ? v : vzero(T());
     }
     if constexpr (APPLY) {
-        __syncthreads();
-        int q0 = 0;
-        for (int ii = i0; ii < i1; ++ii) {
-            const int im = tab.atom_img_list[ii];
-            const int ndc = tab.img_ndc[im];
-            const int nst = (ndc + 31) >> 5;
-            const int* gp = tab.gpos + tab.img_goff[im];
-            const S* ch = chi + tab.img_chi_off[im];
-            for (int s = (w - q0) & 7; s < nst; s += 8) {
-                const int g = 32 * s + lane;
-                if (g >= ndc) break;
-                T* o = out + gp[g];
-                T old[NC], v[NC];
+        q0 = 0;
+        for (int ic = i0; ic < i1; ic += kAtomImgs) {
+            if (i1 - i0 > kAtomImgs) images(ic);  // otherwise still in place
+            else __syncthreads();                  // al
+            const int ni = min(kAtomImgs, i1 - ic);
+            for (int ii = 0; ii < ni; ++ii) {
+                const int ndc = im_ndc[ii];
+                const int nst = (ndc + 31) >> 5;
+                const int* gp = im_gp[ii];
+                const S* ch = im_ch[ii];
+                for (int s = (w - q0) & 7; s < nst; s += 8) {
+                    const int g = 32 * s + lane;
+                    if (g >= ndc) break;
+                    T* o = out + gp[g];
+                    T old[NC], v[NC];
 #pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    old[c] = o[(long long)min(n0 + c, ncol - 1) * ldo];
-                    v[c] = vzero(T());
-                }
+                    for (int c = 0; c < NC; ++c) {
+                        old[c] = o[(long long)min(n0 + c, ncol - 1) * ldo];
+                        v[c] = vzero(T());
+                    }
 #pragma unroll
-                for (int j = 0; j < NP; ++j) {
-                    if (j < np) {
-                        const S cv = ch[(long long)j * ndc + g];
+                    for (int j = 0; j < NP; ++j) {
+                        if (j < np) {
+                            const S cv = ch[(long long)j * ndc + g];
 #pragma unroll
-                        for (int c = 0; c < NC; ++c) v[c] = fmac(v[c], cv, al[j * NC + c]);
+                            for (int c = 0; c < NC; ++c) v[c] = fmac(v[c], cv, al[j * NC + c]);
+                        }
+                    }
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        if constexpr (ScalarOf<T>::cplx) {  // conj of the gather phase: e^{+i k.R_img}
+                            T ph;
+                            ph.x = (S)im_ph[ii].x;
+                            ph.y = -(S)im_ph[ii].y;
+                            v[c] = pmul(v[c], ph);
+                        }
+                        if (n0 + c < ncol) o[(long long)(n0 + c) * ldo] = fmac(old[c], scale, v[c]);
                     }
                 }
-#pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    if constexpr (ScalarOf<T>::cplx) {  // conj of the gather phase: e^{+i k.R_img}
-                        T ph;
-                        ph.x = (S)tab.img_phase[2 * im];
-                        ph.y = -(S)tab.img_phase[2 * im + 1];
-                        v[c] = pmul(v[c], ph);
-                    }
-                    if (n0 + c < ncol) o[(long long)(n0 + c) * ldo] = fmac(old[c], scale, v[c]);
-                }
+                q0 += nst;
             }
-            q0 += nst;
         }
     }
 }
@@ -347,8 +361,9 @@ struct Gather2Geom {
     static constexpr size_t cs_elems = (size_t)kNL2Pts * CSP;
     static constexpr size_t buf_elems = xs_elems + cs_elems;        // one tile buffer
     static constexpr size_t red_elems = (size_t)4 * 32 * 4 * NPG;  // 4 warps x 32 lanes x accumulators
-    static constexpr size_t smem_bytes =
-        sizeof(T) * ((2 * buf_elems) > red_elems ? (2 * buf_elems) : red_elems);
+    static constexpr size_t smem_bytes(int stages) {
+        return sizeof(T) * ((stages * buf_elems) > red_elems ? (stages * buf_elems) : red_elems);
+    }
 };
 
 // Asynchronous 4- or 8-byte global -> shared copy; src_bytes = 0 fills the destination with
@@ -366,21 +381,27 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// Position in an atom's tile sequence: image ii of the atom, first point g0 of the tile.
+// Position in an atom's tile sequence: entry ii of the atom's image list, first point g0 of the tile,
+// and the image's point count and tables.
+template <typename T>
 struct TileIt {
-    int ii, g0;
+    int ii, g0, ndc;
+    const int* gp;
+    const T* ch;
 };
 
-// Tiles are double-buffered: the asynchronous copies of tile t+1 are issued before the FMAs of
-// tile t, so the gathered loads of one tile overlap the arithmetic of the previous one.
-template <typename T, int NPG>
+// Tiles go through a ring of NS buffers: the asynchronous copies of the next NS - 1 tiles are in flight
+// while a tile is multiplied.  With few CTAs (Si64 at 160 states: 192) an atom's chain of tiles is what
+// the launch takes, so they run four buffers (64 -> 59 us a launch); with many (Si216 at 520: 1944)
+// the CTAs resident on an SM hide each other's copies, and two buffers leave room for more of them.
+template <typename T, int NPG, int NS>
 __global__ void __launch_bounds__(256)
     nl_gather2_kernel(const T* __restrict__ x, long long ld, int ncol, int ncolp, NLView tab, T* __restrict__ alpha,
                       double dV) {
     using Geo = Gather2Geom<T, NPG>;
     constexpr int NB = kNL2Cols, G = kNL2Pts, NPGP = Geo::NPGP, CSP = Geo::CSP;
     extern __shared__ __align__(16) unsigned char smraw[];
-    // two tile buffers, each [G][NB] x (4-column groups swizzled by g & 7) then [G][CSP] chi
+    // tile buffers, each [G][NB] x (4-column groups swizzled by g & 7) then [G][CSP] chi
     T* const buf0 = reinterpret_cast<T*>(smraw);
     const T* chi = reinterpret_cast<const T*>(tab.chi);
     const int a = blockIdx.x;
@@ -396,26 +417,47 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
         for (int m = 0; m < NPG; ++m) acc[k][m] = T(0);
 
-    auto normalize = [&](TileIt t) {  // first non-empty tile at or after (ii, g0)
-        while (t.ii < ii_end && t.g0 >= tab.img_ndc[tab.atom_img_list[t.ii]]) {
+    auto open = [&](TileIt<T> t) {  // first non-empty image at or after entry ii
+        for (; t.ii < ii_end; ++t.ii) {
+            const int im = tab.atom_img_list[t.ii];
+            t.ndc = tab.img_ndc[im];
+            if (t.ndc > 0) {
+                t.gp = tab.gpos + tab.img_goff[im];
+                t.ch = chi + tab.img_chi_off[im];
+                break;
+            }
+        }
+        t.g0 = 0;
+        return t;
+    };
+    auto advance = [&](TileIt<T> t) {
+        t.g0 += G;
+        if (t.g0 >= t.ndc) {
             ++t.ii;
-            t.g0 = 0;
+            t = open(t);
         }
         return t;
     };
-    auto issue = [&](TileIt t, int bi) {  // asynchronous copies of tile t into buffer bi
+    // grid positions of the lane's two points of a tile: loaded one tile before the copies that need
+    // them, so that these do not wait for them
+    int pos[2];
+    auto fetch_pos = [&](const TileIt<T>& t) {
+#pragma unroll
+        for (int pp = 0; pp < 2; ++pp) {
+            const int g = t.g0 + lane + 32 * pp;
+            pos[pp] = (t.ii < ii_end && g < t.ndc) ? t.gp[g] : -1;
+        }
+    };
+    auto issue = [&](const TileIt<T>& t, int bi) {  // asynchronous copies of tile t into buffer bi
         T* xs = buf0 + (size_t)bi * Geo::buf_elems;
         T* cs = xs + Geo::xs_elems;
-        const int im = tab.atom_img_list[t.ii];
-        const int ndc = tab.img_ndc[im];
-        const int gl = min(G, ndc - t.g0);
-        const int* gp = tab.gpos + tab.img_goff[im] + t.g0;
-        const T* ch = chi + tab.img_chi_off[im] + t.g0;
+        const int gl = min(G, t.ndc - t.g0);
+        const T* ch = t.ch + t.g0;
 #pragma unroll
         for (int pp = 0; pp < 2; ++pp) {
             const int g = lane + 32 * pp;
-            const bool okg = g < gl;
-            const long long base = okg ? (long long)gp[g] : 0;
+            const bool okg = pos[pp] >= 0;
+            const long long base = okg ? pos[pp] : 0;
 #pragma unroll
             for (int qq = 0; qq < 2; ++qq) {
                 const int q = w + 8 * qq;
@@ -434,25 +476,37 @@ __global__ void __launch_bounds__(256)
             const int gq = sl / NPGP, m = sl % NPGP;
             const int j = gq * NPG + m;
             const bool ok = g < gl && m < NPG && j < np;
-            cp_async_small<sizeof(T)>(cs + g * CSP + sl, ch + (ok ? (long long)j * ndc + g : 0),
+            cp_async_small<sizeof(T)>(cs + g * CSP + sl, ch + (ok ? (long long)j * t.ndc + g : 0),
                                       ok ? (int)sizeof(T) : 0);
         }
         cp_async_commit();
     };
 
-    TileIt cur = normalize(TileIt{tab.atom_img_ptr[a], 0});
-    int bi = 0;
-    if (cur.ii < ii_end) issue(cur, 0);
-    while (cur.ii < ii_end) {
-        const int gl = min(G, tab.img_ndc[tab.atom_img_list[cur.ii]] - cur.g0);
-        const TileIt nxt = normalize(TileIt{cur.ii, cur.g0 + G});
+    TileIt<T> cur = open(TileIt<T>{tab.atom_img_ptr[a], 0, 0, nullptr, nullptr});
+    TileIt<T> nxt = cur;  // the next tile to copy
+    fetch_pos(nxt);
+#pragma unroll
+    for (int s = 0; s < NS - 1; ++s) {
         if (nxt.ii < ii_end) {
-            issue(nxt, bi ^ 1);  // that buffer was released by the barrier that ended the last tile
-            cp_async_wait<1>();
+            issue(nxt, s);
+            nxt = advance(nxt);
+            fetch_pos(nxt);
         } else {
-            cp_async_wait<0>();
+            cp_async_commit();  // one group per stage, empty or not
         }
-        __syncthreads();
+    }
+    int bi = 0;
+    while (cur.ii < ii_end) {
+        const int gl = min(G, cur.ndc - cur.g0);
+        cp_async_wait<NS - 2>();
+        __syncthreads();  // the tile has landed for every warp, and every warp is done with the one before
+        if (nxt.ii < ii_end) {
+            issue(nxt, bi == 0 ? NS - 1 : bi - 1);  // into the buffer of the tile before
+            nxt = advance(nxt);
+            fetch_pos(nxt);
+        } else {
+            cp_async_commit();
+        }
         const T* xs = buf0 + (size_t)bi * Geo::buf_elems;
         const T* cs = xs + Geo::xs_elems;
         for (int g = w; g < gl; g += 8) {
@@ -482,9 +536,8 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
                 for (int m = 0; m < NPG; ++m) acc[k][m] = fma(cv[m], xv[k], acc[k][m]);
         }
-        __syncthreads();  // every warp is done with buffer bi before it is refilled
-        cur = nxt;
-        bi ^= 1;
+        cur = advance(cur);
+        bi = bi + 1 == NS ? 0 : bi + 1;
     }
     // fixed-order tree over the 8 warps: 4+4, 2+2, 1+1
     T* red = reinterpret_cast<T*>(smraw);

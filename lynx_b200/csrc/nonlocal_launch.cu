@@ -45,11 +45,16 @@ int launch_status(const char* what) {
 
 template <typename T, int NPG>
 int gather2(const NLDev& nl, const T* x, long long ld, int ncol, T* alpha, int ncolp, double dV, cudaStream_t st) {
-    const size_t smem = Gather2Geom<T, NPG>::smem_bytes;
-    auto kern = nl_gather2_kernel<T, NPG>;
-    LYNX_CUDA_TRY(smem_cap(kern, smem));
     dim3 grid(nl.n_atom, (ncol + kNL2Cols - 1) / kNL2Cols);
-    kern<<<grid, 256, smem, st>>>(x, ld, ncol, ncolp, make_view<T>(nl), alpha, dV);
+    auto go = [&](auto kern, int stages) -> int {
+        const size_t smem = Gather2Geom<T, NPG>::smem_bytes(stages);
+        LYNX_CUDA_TRY(smem_cap(kern, smem));
+        kern<<<grid, 256, smem, st>>>(x, ld, ncol, ncolp, make_view<T>(nl), alpha, dV);
+        return LYNX_OK;
+    };
+    constexpr int deep = sizeof(T) == 4 ? 4 : 3;
+    if ((long long)grid.x * grid.y <= 4 * 148) LYNX_TRY(go(nl_gather2_kernel<T, NPG, deep>, deep));
+    else LYNX_TRY(go(nl_gather2_kernel<T, NPG, 2>, 2));
     count_launch();
     return launch_status("nonlocal gather");
 }
@@ -77,7 +82,7 @@ int launch_atom_kernel(const NLDev& nl, const T* x, long long ld, int ncol, T* a
                        long long ldo, typename ScalarOf<T>::type scale, cudaStream_t st) {
     auto go = [&](auto kern, int nc) {
         dim3 grid(((APPLY ? ncol : ncolp) + nc - 1) / nc, nl.n_atom);
-        kern<<<grid, 256, 0, st>>>(x, ld, ncol, ncolp, make_view<T>(nl), alpha, dV, out, ldo, scale);
+        launch_pdl(kern, grid, 256, 0, st, x, ld, ncol, ncolp, make_view<T>(nl), alpha, dV, out, ldo, scale);
     };
     constexpr int NC = std::is_same<T, float>::value ? 4 : std::is_same<T, double>::value ? 2 : 1;
     constexpr int NC32 = NC >= 2 ? NC / 2 : 1;

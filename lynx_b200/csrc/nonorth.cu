@@ -68,23 +68,23 @@ __global__ void __launch_bounds__(256)
     gz[o] = sz;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256)
+template <typename T, int R>  // R: the half-width (unrolled: all 6 R loads in flight)
+__global__ void __launch_bounds__(128)
     nonorth_mixed_kernel(const T* __restrict__ gy, const T* __restrict__ gz, long long ldg, T* __restrict__ out,
                          long long ldout, typename ScalarOf<T>::type scale, const NOArgs<T> A) {
-    const long long np = (long long)A.nx * A.ny * A.nz;
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    pdl_wait();
+    const int np = A.nx * A.ny * A.nz;
+    const int t = blockIdx.x * 128 + threadIdx.x;
     if (t >= np) return;
     const int col = blockIdx.y;
-    const int i = (int)(t % A.nx);
-    const int j = (int)((t / A.nx) % A.ny);
-    const int k = (int)(t / ((long long)A.nx * A.ny));
+    const int row = t / A.nx, i = t - row * A.nx, k = row / A.ny, j = row - k * A.ny;
     const T* gyb = gy + (long long)col * ldg;
     const T* gzb = gz + (long long)col * ldg;
-    auto at = [&](int ii, int jj, int kk) { return (long long)ii + (long long)A.nxp * (jj + (long long)A.ny * kk); };
+    auto at = [&](int ii, int jj, int kk) { return ii + A.nxp * (jj + A.ny * kk); };
     using S = typename ScalarOf<T>::type;
     T m = vzero(T());
-    for (int p = 1; p <= A.R; ++p) {
+#pragma unroll
+    for (int p = 1; p <= R; ++p) {
         int ip = i + p, im = i - p;
         const bool rx = ip >= A.nx, lx = im < 0;
         ip -= rx ? A.nx : 0;
@@ -144,7 +144,18 @@ int launch_nonorth_terms(const NonOrthGeom& g, int nxp, const T* x, long long ld
     const long long np = (long long)g.nx * g.ny * g.nz;
     dim3 grid((unsigned)((np + 255) / 256), ncol);
     if (!have_grads) nonorth_grad_kernel<T><<<grid, 256, 0, st>>>(x, ldx, gy, gz, ldg, A);
-    nonorth_mixed_kernel<T><<<grid, 256, 0, st>>>(gy, gz, ldg, out, ldout, (S)(-0.5 * a), A);
+    const dim3 mgrid((unsigned)((np + 127) / 128), ncol);
+    auto mixed = [&](auto kern) { launch_pdl(kern, mgrid, 128, 0, st, gy, gz, ldg, out, ldout, (S)(-0.5 * a), A); };
+    switch (g.R) {
+        case 1: mixed(nonorth_mixed_kernel<T, 1>); break;
+        case 2: mixed(nonorth_mixed_kernel<T, 2>); break;
+        case 3: mixed(nonorth_mixed_kernel<T, 3>); break;
+        case 4: mixed(nonorth_mixed_kernel<T, 4>); break;
+        case 5: mixed(nonorth_mixed_kernel<T, 5>); break;
+        case 6: mixed(nonorth_mixed_kernel<T, 6>); break;
+        case 7: mixed(nonorth_mixed_kernel<T, 7>); break;
+        case 8: mixed(nonorth_mixed_kernel<T, 8>); break;
+    }
     count_launch(have_grads ? 1 : 2);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {

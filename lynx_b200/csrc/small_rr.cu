@@ -49,7 +49,19 @@ __device__ __forceinline__ double2 cj(double2 a) { return make_double2(a.x, -a.y
 __device__ __forceinline__ double re(double a) { return a; }
 __device__ __forceinline__ double re(double2 a) { return a.x; }
 __device__ __forceinline__ double mod(double a) { return fabs(a); }
-__device__ __forceinline__ double mod(double2 a) { return hypot(a.x, a.y); }
+__device__ __forceinline__ double mod(double2 a) { return sqrt(fma(a.x, a.x, a.y * a.y)); }
+// |a|, and e = a / |a| (1 for a = 0)
+__device__ __forceinline__ double mod_phase(double a, double& e) {
+    e = a < 0.0 ? -1.0 : 1.0;
+    return fabs(a);
+}
+__device__ __forceinline__ double mod_phase(double2 a, double2& e) {
+    const double s = fma(a.x, a.x, a.y * a.y);
+    if (!(s > 0x1p-900)) return 0.0;
+    const double r = rsqrt(s);
+    e = make_double2(a.x * r, a.y * r);
+    return s * r;
+}
 __device__ __forceinline__ bool fin(double a) { return isfinite(a); }
 __device__ __forceinline__ bool fin(double2 a) { return isfinite(a.x) && isfinite(a.y); }
 __device__ __forceinline__ void set_re(double& a, double v) { a = v; }
@@ -168,8 +180,8 @@ __global__ void __launch_bounds__(kEigThreads)
     W* V = A + n2;
     W* ph = V + n2;                                   // [NP/2] phase of the pair's entry
     double* cs = reinterpret_cast<double*>(ph + NP / 2);  // [NP/2][2] cosine, sine
-    double* dg = cs + NP;                             // [NP/2][2] new diagonal entries
-    double* red = dg + NP;                            // [kEigThreads / 32]
+    double* dg = cs + NP;                             // [NP/2][3] new diagonal and off-diagonal entries
+    double* red = dg + NP + NP / 2;                            // [kEigThreads / 32]
     int* pq = reinterpret_cast<int*>(red + kEigThreads / 32);  // [NP/2][2] rows of the pair (p < 0: idle)
     int* rank = pq + NP;                              // [N]
     __shared__ int bad, chol, moved;
@@ -254,13 +266,19 @@ __global__ void __launch_bounds__(kEigThreads)
     __syncthreads();
     nrm = 0.0;
     for (int w = 0; w < kEigThreads / 32; ++w) nrm += red[w];
-    const double thr = 0x1p-54 * sqrt(nrm);
+    const double thr = 0x1p-54 * sqrt(nrm), inv = nrm > 0.0 ? rsqrt(nrm) : 0.0;
     // Jacobi sweeps
     const int np2 = NP / 2;
     bool done = false;
     for (int sweep = 0; sweep < kMaxSweeps && !done; ++sweep) {
-        __syncthreads();
+        // done when nothing is left to rotate
         if (tid == 0) moved = 0;
+        __syncthreads();
+        for (int e = tid; e < n2; e += kEigThreads)
+            if (e % N < e / N && mod(A[e]) > thr) moved = 1;
+        __syncthreads();
+        done = moved == 0;
+        if (done) break;
         for (int rnd = 0; rnd < NP - 1; ++rnd) {
             __syncthreads();
             if (tid < np2) {
@@ -276,19 +294,26 @@ __global__ void __launch_bounds__(kEigThreads)
                 set_re(e, 1.0);
                 const bool idle = q >= N;
                 if (!idle) {
+                    // t = tan of the angle that zeroes the entry, 2 m / (d + sign(d) sqrt(d^2 + 4 m^2)), d = aqq -
+                    // app.  An FP32 angle does: the rotation is orthogonal to FP64 for any t, and what
+                    // is left of the entry, 1e-7 of it, goes in the next sweep (FP64 divisions and square
+                    // roots one after another were most of a round's time).
                     const W apq = A[p + q * N];
-                    const double app = re(A[p + p * N]), aqq = re(A[q + q * N]), m = mod(apq);
-                    dg[2 * tid] = app;
-                    dg[2 * tid + 1] = aqq;
+                    const double app = re(A[p + p * N]), aqq = re(A[q + q * N]);
+                    const double m = mod_phase(apq, e), d = aqq - app;
+                    dg[3 * tid] = app;
+                    dg[3 * tid + 1] = aqq;
                     if (m > thr) {
-                        const double th = (aqq - app) / (2.0 * m);
-                        const double t = (th >= 0.0 ? 1.0 : -1.0) / (fabs(th) + sqrt(fma(th, th, 1.0)));
-                        c = 1.0 / sqrt(fma(t, t, 1.0));
+                        const float ms = (float)(m * inv), ds = (float)(d * inv);
+                        const double t = 2.0f * ms / (ds + copysignf(sqrtf(fmaf(ds, ds, 4.0f * ms * ms)), ds));
+                        const double c2 = 1.0 / fma(t, t, 1.0);
+                        c = rsqrt(fma(t, t, 1.0));
                         s = t * c;
-                        e = vscale(1.0 / m, apq);
-                        dg[2 * tid] = app - t * m;
-                        dg[2 * tid + 1] = aqq + t * m;
-                        moved = 1;
+                        dg[3 * tid] = fma(c2 * t, fma(t, d, -2.0 * m), app);
+                        dg[3 * tid + 1] = fma(-c2 * t, fma(t, d, -2.0 * m), aqq);
+                        dg[3 * tid + 2] = c2 * (m - t * fma(m, t, d));
+                    } else {
+                        set_re(e, 1.0);  // not rotated: no phase either
                     }
                 }
                 cs[2 * tid] = c;
@@ -308,9 +333,10 @@ __global__ void __launch_bounds__(kEigThreads)
                     const double c2 = cs[2 * Q], s2 = v2 ? cs[2 * Q + 1] : 0.0;
                     if (s1 == 0.0 && s2 == 0.0) continue;
                     if (P == Q) {
-                        set_re(A[p1 + p1 * N], dg[2 * P]);
-                        set_re(A[q1 + q1 * N], dg[2 * P + 1]);
-                        A[p1 + q1 * N] = A[q1 + p1 * N] = vzero(W());
+                        set_re(A[p1 + p1 * N], dg[3 * P]);
+                        set_re(A[q1 + q1 * N], dg[3 * P + 1]);
+                        set_re(A[p1 + q1 * N], dg[3 * P + 2]);
+                        A[q1 + p1 * N] = A[p1 + q1 * N];
                         continue;
                     }
                     const W z = vzero(W());
@@ -342,7 +368,6 @@ __global__ void __launch_bounds__(kEigThreads)
             }
         }
         __syncthreads();
-        done = moved == 0;
     }
     if (!done) {
         if (tid == 0) info[1] = 1;
@@ -430,7 +455,7 @@ int launch_small_rr(const T* Y, const T* HY, long long ld, long long rows, int n
     LYNX_CUDA_TRY(smem_cap(small_gram_kernel<T>, sg));
     small_gram_kernel<T><<<nch, 256, sg, st>>>(Y, HY, ld, rows, n, chunk, part);
     small_reduce_kernel<W><<<(2 * n * n * 8 + 255) / 256, 256, 0, st>>>(part, nch, n, dV, ms, hs);
-    const size_t se = sizeof(W) * ((size_t)3 * n * n + np / 2) + sizeof(double) * (2 * np + kEigThreads / 32) +
+    const size_t se = sizeof(W) * ((size_t)3 * n * n + np / 2) + sizeof(double) * (2 * np + np / 2 + kEigThreads / 32) +
                       sizeof(int) * (np + n);
     LYNX_CUDA_TRY(smem_cap(small_eig_kernel<W>, se));
     small_eig_kernel<W><<<1, kEigThreads, se, st>>>(ms, hs, n, eig, info);

@@ -47,6 +47,7 @@ __global__ void __launch_bounds__(128)
                        const typename ScalarOf<T>::type* __restrict__ V, T* __restrict__ gy, T* __restrict__ gz,
                        const DirectArgs<T> A) {
     using S = typename ScalarOf<T>::type;
+    pdl_wait();
     const int t = blockIdx.x * 128 + threadIdx.x;
     if (t >= A.nx * A.ny * A.nz) return;
     const int row = t / A.nx, i = t - row * A.nx;
@@ -160,7 +161,7 @@ int launch_direct_step(const StencilGeom& g, int nxp, const T* x, long long ldx,
         constexpr int R = decltype(rc)::value;
         auto kern = ng ? (xo ? direct_step_kernel<T, R, true, true> : direct_step_kernel<T, R, false, true>)
                        : (xo ? direct_step_kernel<T, R, true, false> : direct_step_kernel<T, R, false, false>);
-        kern<<<grid, 128, 0, st>>>(x, xold, out, V, gy, gz, A);
+        launch_pdl(kern, grid, 128, 0, st, x, xold, out, V, gy, gz, A);
     };
     switch (g.R) {
         case 1: go(std::integral_constant<int, 1>{}); break;
