@@ -133,17 +133,24 @@ __global__ void __launch_bounds__(256)
         }
         __syncthreads();
         const int np0 = min(256, total - p0);
-        for (int q = lane; q < np0; q += 32) {
+        // the projector values of all eight steps of the tile first: their latency is paid once
+        double c[8][MJ];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int q = min(lane + 32 * u, np0 - 1);
             const double* cp = chi + cbase[q];
             const long long st = cstride[q];
-            double c[MJ];
 #pragma unroll
-            for (int m = 0; m < MJ; ++m) c[m] = cp[min(w + 8 * m, np - 1) * st];
+            for (int m = 0; m < MJ; ++m) c[u][m] = lane + 32 * u < np0 ? cp[min(w + 8 * m, np - 1) * st] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int q = min(lane + 32 * u, np0 - 1);
 #pragma unroll
             for (int v = 0; v <= NV; ++v) {
                 const T xv = val[v][q];
 #pragma unroll
-                for (int m = 0; m < MJ; ++m) acc[m][v] = fmac(acc[m][v], c[m], xv);
+                for (int m = 0; m < MJ; ++m) acc[m][v] = fmac(acc[m][v], c[u][m], xv);
             }
         }
     }
@@ -198,7 +205,8 @@ __global__ void __launch_bounds__(256)
 // points of Re(conj(g_a) g_b).  CTA = a band of rows of one column and a chunk of planes; a thread
 // owns two rows' points at one x and marches through z with the 2 R + 1 planes of its points in
 // registers (complex: one row's); the plane's rows with R halo rows on either side are staged in shared memory for the x
-// and y neighbours (two buffers: the next plane's copies overlap this plane's sums).
+// and y neighbours (three buffers: the copies of the next two planes overlap this plane's sums, and one
+// barrier a plane suffices).
 constexpr int kKinThreads = 512;
 template <typename T> constexpr int kin_ry() { return ScalarOf<T>::cplx ? 1 : 2; }  // window registers
 template <typename T, int R, bool PH>
@@ -207,7 +215,7 @@ __global__ void __launch_bounds__(kKinThreads, 1)
                    double* __restrict__ part) {
     constexpr int RY = kin_ry<T>(), W = 2 * R + 1;
     extern __shared__ __align__(16) unsigned char sm_raw[];
-    T* tile = reinterpret_cast<T*>(sm_raw);  // [2][TY + 2R][nx]
+    T* tile = reinterpret_cast<T*>(sm_raw);  // [3][TY + 2R][nx]
     __shared__ double red[kKinThreads / 32][6];
     const int nx = G.nx, ny = G.ny, nz = G.nz, tid = threadIdx.x;
     const int TY = tyt * RY, rows = TY + 2 * R;
@@ -252,18 +260,17 @@ __global__ void __launch_bounds__(kKinThreads, 1)
         for (int r = 0; r < RY; ++r) win[k][r] = load(z0 - R + k, r);
     double s[6] = {0, 0, 0, 0, 0, 0};
     stage(z0, 0);
+    if (z0 + 1 < z1) stage(z0 + 1, 1);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
+    int b = 0;
     for (int z = z0; z < z1; ++z) {
-        const int b = (z - z0) & 1;
         T nxt[RY];
-        if (z + 1 < z1) {
-            stage(z + 1, b ^ 1);  // that buffer was released by the barrier that ended the last plane
 #pragma unroll
-            for (int r = 0; r < RY; ++r) nxt[r] = load(z + R + 1, r);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
-        __syncthreads();
+        for (int r = 0; r < RY; ++r) nxt[r] = z + 1 < z1 ? load(z + R + 1, r) : vzero(T());
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();  // the plane has landed, and every thread is done with the one before
+        if (z + 2 < z1) stage(z + 2, b == 0 ? 2 : b - 1);
+        else asm volatile("cp.async.commit_group;" ::: "memory");
         const T* tl = tile + (size_t)b * rows * nx;
 #pragma unroll
         for (int r = 0; r < RY; ++r) {
@@ -307,7 +314,7 @@ __global__ void __launch_bounds__(kKinThreads, 1)
             for (int r = 0; r < RY; ++r) win[k][r] = win[k + 1][r];
 #pragma unroll
         for (int r = 0; r < RY; ++r) win[W - 1][r] = nxt[r];
-        __syncthreads();
+        b = b == 2 ? 0 : b + 1;
     }
 #pragma unroll
     for (int v = 0; v < 6; ++v) {
@@ -515,7 +522,7 @@ int launch_kinetic(const ForceGeom& g, const T* psi, long long ld, int ncol, con
     const GradCoef<T> G = grad_coef<T>(g, phl, phr);
     constexpr int ry = kin_ry<T>();
     const KinPlan k = kin_plan(g, ncol, ry);
-    const size_t smem = sizeof(T) * 2 * (size_t)(k.tyt * ry + 2 * g.R) * g.nx;
+    const size_t smem = sizeof(T) * 3 * (size_t)(k.tyt * ry + 2 * g.R) * g.nx;
     if (g.nx > kKinThreads || smem > 200 * 1024) {
         kinetic_point_kernel<T><<<dim3(kPointCtas, ncol), 256, 0, st>>>(psi, ld, G, work);
         kinetic_reduce_kernel<<<6, 256, 0, st>>>(work, occ, ncol, kPointCtas, scale, out);
