@@ -849,6 +849,7 @@ __global__ void __launch_bounds__(kExpThreads)
 // projector count), the order of the kernels above: bitwise their results.  FP32 column pairs
 // use packed fma.rn.f32x2, element for element the same rounding.
 constexpr int kExpRegCols = 32;
+constexpr int kExpMaxAtoms = 64;  // most atoms of a tile that the kernel takes
 template <typename T>
 constexpr int exp_reg_threads() {
     return kExpTilePts / (16 / (int)sizeof(T));
@@ -873,20 +874,26 @@ __global__ void __launch_bounds__(exp_reg_threads<T>())
     V16* al_s = reinterpret_cast<V16*>(smx);
     const int t = blockIdx.x, tid = threadIdx.x;
     const int c0 = blockIdx.y * kExpRegCols;
-    const int* ta = tile_atoms + (long long)t * amax;
+    // the tile's atoms first, then every alpha vector as an asynchronous copy (all in flight at once,
+    // while the projector values are loaded below); rows and columns that do not exist become zeros
+    __shared__ int2 at_s[kExpMaxAtoms];  // first projector row, projector count
+    for (int i = tid; i < amax; i += NT) {
+        const int a = tile_atoms[(long long)t * amax + i];
+        at_s[i] = a >= 0 ? make_int2(atom_poff[a], atom_nproj[a]) : make_int2(0, 0);
+    }
+    __syncthreads();
     for (int e = tid; e < amax * NP * NV; e += NT) {
         const int r = e / NV, v = e - r * NV;
         const int slot = r / NP, j = r - slot * NP;
-        const int a = ta[slot];
+        const int2 at = at_s[slot];
         const int col = c0 + v * VW;
-        V16 val;
-        T* vp = reinterpret_cast<T*>(&val);
-#pragma unroll
-        for (int c = 0; c < VW; ++c) vp[c] = T(0);
-        if (a >= 0 && j < atom_nproj[a] && col < ncolp)
-            val = *reinterpret_cast<const V16*>(alpha + (long long)(atom_poff[a] + j) * ncolp + col);
-        al_s[slot * SS + j * NV + v] = val;
+        const bool ok = j < at.y && col < ncolp;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                         static_cast<uint32_t>(__cvta_generic_to_shared(al_s + slot * SS + j * NV + v))),
+                     "l"(alpha + (ok ? (long long)(at.x + j) * ncolp + col : 0)), "r"(ok ? 16 : 0)
+                     : "memory");
     }
+    cp_async_commit();
     const long long m0 = (long long)t * kExpTilePts + PTS * tid;
     const int npt = (int)max(0LL, min((long long)PTS, (long long)n_pts - m0));
     T cj[NP][PTS];
@@ -907,6 +914,7 @@ __global__ void __launch_bounds__(exp_reg_threads<T>())
     int so[PTS];  // each point's slot row in al_s (past the last point: the previous one's)
 #pragma unroll
     for (int k = 0; k < PTS; ++k) so[k] = (k < npt) ? (int)pt_slot[m0 + k] * SS : (k > 0 ? so[k - 1] : 0);
+    cp_async_wait<0>();
     __syncthreads();  // alpha staged
     if (npt == 0) return;
 #pragma unroll 1

@@ -178,7 +178,7 @@ int launch_nl_expand(const NLDev& nl, T* W, long long ldw, int ncol, const T* al
         const size_t nrow = (size_t)nl.exp_amax * NP;
         const size_t smem = (size_t)NP * kExpTilePts * sizeof(T) + 2 * nrow * 16;
         const size_t smem_reg = (size_t)nl.exp_amax * (NP * kExpRegCols * sizeof(T) + 16);
-        if (NP <= 18 && nl.exp_tile_atoms && smem_reg <= 96 * 1024 && (ldw % 4) == 0) {
+        if (NP <= 18 && nl.exp_tile_atoms && nl.exp_amax <= kExpMaxAtoms && smem_reg <= 96 * 1024 && (ldw % 4) == 0) {
             // projector values in registers (up to 18 per point), alpha staged in shared memory
             dim3 grid((nl.n_pts + kExpTilePts - 1) / kExpTilePts, (ncol + kExpRegCols - 1) / kExpRegCols);
             auto go = [&](auto kern) -> int {
