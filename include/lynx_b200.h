@@ -281,6 +281,10 @@ LYNX_API int lynx_rotate_mixed(lynx_ctx* ctx, const float* Y, long long ld, long
 LYNX_API int lynx_electron_density(lynx_ctx* ctx, const double* psi, int nband, int ld, const double* occ,
                                    double weight, double* rho, int is_complex, int accumulate);
 
+/* out[i] = sum_n u_n(i) v_n(i) over ncol real columns (stride ld), Nd values: the gradient of
+ * sum_n <u_n, H v_n> in the potential.  No counterpart in the reference. */
+LYNX_API int lynx_pair_density(lynx_ctx* ctx, const double* u, const double* v, int ncol, int ld, double* out);
+
 /* One CheFSI pass of real orbitals, as lynx_eigensolver_solve, for a system of one spin channel and
  * one k-point, followed by the next steps of the SCF iteration on its Ritz values: the Fermi level
  * (Brent on sum_n weight f(eig_n - Ef) = nelectron, smearing as lynx_fermi_level), the

@@ -65,7 +65,12 @@ def _make_fns():
             psi, veff = fctx.saved_tensors
             g = grad_y.contiguous()
             grad_psi = solver.Hamiltonian(fctx.ctx).apply(g, Veff=veff.contiguous()) if fctx.needs_input_grad[0] else None
-            grad_v = (g * psi).sum(0) if fctx.needs_input_grad[1] else None
+            grad_v = None
+            if fctx.needs_input_grad[1]:
+                # one kernel, unless this backward is itself recorded (create_graph) or the block is one
+                # vector: then torch's own operations
+                plain = not torch.is_grad_enabled() and psi.dim() == 2 and psi.dtype == torch.float64 and psi.is_cuda
+                grad_v = solver.pair_density(fctx.ctx, g, psi.contiguous()) if plain else (g * psi).sum(0)
             grad_pos = None
             if fctx.needs_input_grad[2]:
                 ones = np.ones(psi.shape[0])

@@ -246,6 +246,29 @@ template int launch_density<double>(const double*, long long, long long, int, co
 template int launch_density<double2>(const double2*, long long, long long, int, const double*, double*, bool,
                                      cudaStream_t);
 
+// out[i] = sum_n u_n(i) v_n(i), the columns in order: one read of both blocks (the gradient of <g, H psi>
+// in the potential; as a product block and a sum of it, 161 us at Si64 with 160 states, 94 us here).
+// V: points per thread, loaded as one vector.
+template <int V>
+__global__ void __launch_bounds__(128)
+    pair_density_kernel(const double* __restrict__ u, const double* __restrict__ v, long long ld, long long nd,
+                        int ncol, double* __restrict__ out) {
+    using T = typename std::conditional<V == 2, double2, double>::type;
+    const long long i = (blockIdx.x * 128LL + threadIdx.x) * V;
+    if (i >= nd) return;
+    double s[V] = {};
+#pragma unroll 8
+    for (int n = 0; n < ncol; ++n) {
+        const T a = __ldcs(reinterpret_cast<const T*>(u + n * ld + i)), b = __ldcs(reinterpret_cast<const T*>(v + n * ld + i));
+        const double* ap = reinterpret_cast<const double*>(&a);
+        const double* bp = reinterpret_cast<const double*>(&b);
+#pragma unroll
+        for (int q = 0; q < V; ++q) s[q] = fma(ap[q], bp[q], s[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < V; ++q) out[i + q] = s[q];
+}
+
 // Sets *flag when an entry of the N x N column-major matrix A is NaN or Inf (comps doubles per
 // entry: 1 real, 2 complex; upper: only entries on or above the diagonal are valid).
 __global__ void nonfinite_kernel(const double* __restrict__ A, int N, int comps, int upper, int* __restrict__ flag) {
@@ -2604,6 +2627,22 @@ extern "C" int lynx_electron_density(lynx_ctx* c, const double* psi, int nband, 
         LYNX_TRY(launch_density<double>(psi, l, c->Nd, nband, c->dens_w.as<double>(), rho, accumulate != 0,
                                         c->stream));
     LYNX_CUDA_TRY(cudaStreamSynchronize(c->stream));  // w is a host temporary
+    return LYNX_OK;
+}
+
+extern "C" int lynx_pair_density(lynx_ctx* c, const double* u, const double* v, int ncol, int ld, double* out) {
+    LYNX_CHECK_ARG(c && u && v && out, "null pointer");
+    LYNX_CHECK_ARG(ncol > 0, "ncol must be positive");
+    const long long l = ld > 0 ? ld : c->Nd, nd = c->Nd;
+    LYNX_CHECK_ARG(l >= nd, "ld < Nd");
+    LYNX_TRY(activate(c));
+    const bool pairs = nd % 2 == 0 && l % 2 == 0 && aligned16(u) && aligned16(v);
+    if (pairs)
+        pair_density_kernel<2><<<(unsigned)((nd / 2 + 127) / 128), 128, 0, c->stream>>>(u, v, l, nd, ncol, out);
+    else
+        pair_density_kernel<1><<<(unsigned)((nd + 127) / 128), 128, 0, c->stream>>>(u, v, l, nd, ncol, out);
+    count_launch();
+    LYNX_CUDA_TRY(cudaGetLastError());
     return LYNX_OK;
 }
 

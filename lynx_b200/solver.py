@@ -416,6 +416,15 @@ def electron_density(ctx: Context, psi, occ, weight: float = 2.0, rho=None, comp
     return rho
 
 
+def pair_density(ctx: Context, u, v):
+    """sum_n u_n v_n at every grid point (lynx_pair_density), for device blocks (ncol, Nd), float64."""
+    ctx.sync_stream()
+    out = _torch().empty(ctx.nd, dtype=u.dtype, device=u.device)
+    check(ctx.lib.lynx_pair_density(ctx.handle, ctypes.c_void_p(_dev_ptr(u)), ctypes.c_void_p(_dev_ptr(v)), u.shape[0],
+                                    ctx.nd, ctypes.c_void_p(out.data_ptr())))
+    return out
+
+
 def randomize_orbitals(ctx: Context, nband: int, seed: int, complex_: bool = False):
     """Device start orbitals as EigenSolver::randomize_psi_gpu draws them (cuRAND default
     generator, uniform (0, 1], seed as given): a torch tensor (nband, Nd), float64 or complex128
