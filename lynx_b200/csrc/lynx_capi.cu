@@ -328,7 +328,13 @@ struct lynx_ctx {
     DevBuf lz[4];         // Lanczos vectors
     DevBuf io_psi, io_v;  // staging for the host-pointer solve
     DevBuf vpad64, vpad32;  // Veff in the padded row layouts of the pipelined stencil
-    DevBuf errflag;         // set by a kernel whose bounded wait gave up
+    // Set by a kernel whose bounded wait gave up: an int in mapped host memory, so that looking at it after
+    // a synchronisation is a host read (a copy of 4 bytes to pageable memory cost as much as a small call's
+    // kernel).  Pinned host memory for the results of a pass likewise.
+    int* err_h = nullptr;
+    int* err_d = nullptr;
+    double* res_h = nullptr;
+    size_t res_n = 0;
     DevBuf gwork;           // slices, exponents and split partials of the tensor-core Gram
     DevBuf rwork;           // slices and exponents of the tensor-core rotation
     DevBuf cplx_work;       // planar split and real 2N x 2N products of the mixed k-point Rayleigh-Ritz
@@ -725,13 +731,20 @@ int veff_layout(lynx_ctx* c, const double* v, int nxp, const S** out) {
     return LYNX_OK;
 }
 
+int ensure_errflag(lynx_ctx* c) {
+    if (c->err_h) return LYNX_OK;
+    LYNX_CUDA_TRY(cudaHostAlloc(&c->err_h, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+    *c->err_h = 0;
+    LYNX_CUDA_TRY(cudaHostGetDevicePointer(&c->err_d, c->err_h, 0));
+    return LYNX_OK;
+}
+
 int check_errflag(lynx_ctx* c) {
-    if (!c->errflag.p) return LYNX_OK;
-    int h = 0;
-    LYNX_CUDA_TRY(cudaMemcpyAsync(&h, c->errflag.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    if (!c->err_h) return LYNX_OK;
     LYNX_CUDA_TRY(cudaStreamSynchronize(c->stream));
-    if (h) {
-        cudaMemsetAsync(c->errflag.p, 0, sizeof(int), c->stream);
+    volatile int* flag = c->err_h;
+    if (*flag) {
+        *flag = 0;
         set_error("a bounded device-side wait gave up (shared-memory pipeline did not complete)");
         return LYNX_ERR_TIMEOUT;
     }
@@ -756,12 +769,12 @@ int pipe_launch_tuned(lynx_ctx* c, int nxp, const T* x, long long ldx, const T* 
                                           ncol, nlh != nullptr, xold != nullptr && d != 0.0};
     if (c->force_shape >= 0)
         return launch_cheb_pipe<T, S>(g, nxp, x, ldx, xold, ldo, out, ldout, V, ncol, a, b, d, phl, phr,
-                                      c->errflag.as<int>(), c->stream, c->force_shape < nsh ? c->force_shape : 0, nlh);
+                                      c->err_d, c->stream, c->force_shape < nsh ? c->force_shape : 0, nlh);
     auto it = c->pipe_shape.find(key);
     if (it != c->pipe_shape.end() || nsh <= 1 || !c->autotune) {
         const int si = (it != c->pipe_shape.end()) ? it->second : 0;
         return launch_cheb_pipe<T, S>(g, nxp, x, ldx, xold, ldo, out, ldout, V, ncol, a, b, d, phl, phr,
-                                      c->errflag.as<int>(), c->stream, si, nlh);
+                                      c->err_d, c->stream, si, nlh);
     }
     cudaEvent_t e0, e1;
     LYNX_CUDA_TRY(cudaEventCreate(&e0));
@@ -771,7 +784,7 @@ int pipe_launch_tuned(lynx_ctx* c, int nxp, const T* x, long long ldx, const T* 
     int rc = LYNX_OK;
     for (int si = 0; si < nsh && rc == LYNX_OK; ++si) {
         rc = launch_cheb_pipe<T, S>(g, nxp, x, ldx, xold, ldo, out, ldout, V, ncol, a, b, d, phl, phr,
-                                    c->errflag.as<int>(), c->stream, si, nlh);
+                                    c->err_d, c->stream, si, nlh);
         if (rc == LYNX_ERR_UNSUPPORTED) {  // this shape's stages do not fit: try the others
             rc = LYNX_OK;
             continue;
@@ -779,7 +792,7 @@ int pipe_launch_tuned(lynx_ctx* c, int nxp, const T* x, long long ldx, const T* 
         if (rc != LYNX_OK) break;
         cudaEventRecord(e0, c->stream);
         rc = launch_cheb_pipe<T, S>(g, nxp, x, ldx, xold, ldo, out, ldout, V, ncol, a, b, d, phl, phr,
-                                    c->errflag.as<int>(), c->stream, si, nlh);
+                                    c->err_d, c->stream, si, nlh);
         cudaEventRecord(e1, c->stream);
         if (rc != LYNX_OK) break;
         if (cudaEventSynchronize(e1) != cudaSuccess) {
@@ -804,7 +817,7 @@ int pipe_launch_tuned(lynx_ctx* c, int nxp, const T* x, long long ldx, const T* 
     c->pipe_shape[key] = best;
     // leave the chosen shape's (identical) output as the result of record
     return launch_cheb_pipe<T, S>(g, nxp, x, ldx, xold, ldo, out, ldout, V, ncol, a, b, d, phl, phr,
-                                  c->errflag.as<int>(), c->stream, best, nlh);
+                                  c->err_d, c->stream, best, nlh);
 }
 
 // Adds the duration of the stencil launch bracketed by c->kt[0] (recorded before it) and an event
@@ -889,7 +902,7 @@ int cheb_step(lynx_ctx* c, int nxp, const T* x, long long ldx, const T* xold, lo
     }
     if constexpr (!ScalarOf<T>::cplx) {
         if (!direct) {
-            if (!c->errflag.p) LYNX_TRY(ensure_zeroed(c, c->errflag, sizeof(int)));
+            LYNX_TRY(ensure_errflag(c));
             if (fuse) {
                 const lynx_ctx::NLMap* nm = nullptr;
                 LYNX_TRY(nl_map_for(c, nxp, &nm));
@@ -1082,10 +1095,20 @@ int check_finite(lynx_ctx* c, const double* A, int N, int comps, bool upper, int
 }
 
 int finish_rr(lynx_ctx* c, int N, double* eig_host) {
+    const size_t need = (size_t)N + 2;  // Ritz values, then info
+    if (c->res_n < need) {
+        if (c->res_h) cudaFreeHost(c->res_h);
+        c->res_h = nullptr;
+        c->res_n = 0;
+        LYNX_CUDA_TRY(cudaHostAlloc(&c->res_h, need * sizeof(double), cudaHostAllocPortable));
+        c->res_n = need;
+    }
     int info[3] = {0, 0, 0};
-    LYNX_CUDA_TRY(cudaMemcpyAsync(info, c->info.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    LYNX_CUDA_TRY(cudaMemcpyAsync(eig_host, c->eigd.p, N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    LYNX_CUDA_TRY(cudaMemcpyAsync(c->res_h, c->eigd.p, N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    LYNX_CUDA_TRY(cudaMemcpyAsync(c->res_h + N, c->info.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     LYNX_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    std::memcpy(eig_host, c->res_h, N * sizeof(double));
+    std::memcpy(info, c->res_h + N, 3 * sizeof(int));
     if (info[2] != 0) {
         set_error("non-finite entries in the overlap or projected Hamiltonian (NaN/Inf in the orbitals or Veff)");
         return LYNX_ERR_NONFINITE;
@@ -1199,9 +1222,9 @@ int rayleigh_ritz_mixed_real(lynx_ctx* c, const float* Y32, const float* HY32, l
     LYNX_TRY(rr_alloc_small(c, N, sizeof(double)));
     const GramPlan plan = gram_plan(ldb, N);  // all ldb rows: pad elements are zero
     LYNX_TRY(c->gwork.ensure(plan.work_bytes));
-    if (!c->errflag.p) LYNX_TRY(ensure_zeroed(c, c->errflag, sizeof(int)));
+    LYNX_TRY(ensure_errflag(c));
     LYNX_TRY(launch_gram_i8(Y32, HY32, ldb, ldb, N, c->dV, plan, c->gwork.p, c->gwork.bytes, c->Ms.as<double>(),
-                            c->Hs.as<double>(), c->errflag.as<int>(), c->info.as<int>() + 2, c->stream));
+                            c->Hs.as<double>(), c->err_d, c->info.as<int>() + 2, c->stream));
     if (rot_supported(N)) {
         // rotation on the tensor cores, straight from the FP32 block into the caller's psi
         const RotPlan rp = rot_plan(ldb, N);
@@ -1217,13 +1240,13 @@ int rayleigh_ritz_mixed_real(lynx_ctx* c, const float* Y32, const float* HY32, l
             LYNX_TRY(c->dens_part.ensure(sizeof(double) * (size_t)ntn * c->Nd));
             RotDensity rd{c->dens_w.as<double>(), c->dens_part.as<double>(), c->dens.rho, c->Nd, false};
             LYNX_TRY(launch_rot_i8(Y32, ldb, ldb, c->nx, nxp, c->Hs.as<double>(), N, rp, c->rwork.p, c->rwork.bytes,
-                                   psi, ldp, c->errflag.as<int>(), c->stream, &rd));
+                                   psi, ldp, c->err_d, c->stream, &rd));
             c->dens.done = true;
             LYNX_CUDA_TRY(cudaStreamSynchronize(c->stream));
             return LYNX_OK;
         }
         LYNX_TRY(launch_rot_i8(Y32, ldb, ldb, c->nx, nxp, c->Hs.as<double>(), N, rp, c->rwork.p, c->rwork.bytes, psi,
-                               ldp, c->errflag.as<int>(), c->stream));
+                               ldp, c->err_d, c->stream));
         return finish_rr(c, N, eig_host);
     }
     const long long Nd = c->Nd;
@@ -1321,9 +1344,9 @@ int rayleigh_ritz_mixed_cplx(lynx_ctx* c, const float2* Y32, const float2* HY32,
     count_launch(2);
     const GramPlan plan = gram_plan(ldb, N2);  // all ldb rows: pad elements are zero
     LYNX_TRY(c->gwork.ensure(plan.work_bytes));
-    if (!c->errflag.p) LYNX_TRY(ensure_zeroed(c, c->errflag, sizeof(int)));
+    LYNX_TRY(ensure_errflag(c));
     LYNX_TRY(launch_gram_i8(Yp, Hp, ldb, ldb, N2, c->dV, plan, c->gwork.p, c->gwork.bytes, Mpl, Hpl,
-                            c->errflag.as<int>(), c->info.as<int>() + 2, c->stream));
+                            c->err_d, c->info.as<int>() + 2, c->stream));
     const RotPlan rp = rot_plan(ldb, N2);
     LYNX_TRY(c->rwork.ensure(rp.work_bytes));
     LYNX_TRY(launch_colexp(Mpl, N2, c->rwork.p, rp, ldb, c->stream));  // scaling of the 2N planar states
@@ -1339,7 +1362,7 @@ int rayleigh_ritz_mixed_cplx(lynx_ctx* c, const float2* Y32, const float2* HY32,
         count_launch();
     }
     LYNX_TRY(launch_rot_i8(Yp, ldb, ldb, c->nx, nxp, Wt, N2, rp, c->rwork.p, c->rwork.bytes, R, Nd,
-                           c->errflag.as<int>(), c->stream));
+                           c->err_d, c->stream));
     const int ib = (int)std::min<long long>((Nd * N + 255) / 256, 148LL * 16);
     interleave_kernel<<<ib, 256, 0, c->stream>>>(R, Nd, N, psi, ldp);
     count_launch();
@@ -1726,7 +1749,8 @@ int lynx_destroy(lynx_ctx* c) {
     c->io_v.release();
     c->vpad64.release();
     c->vpad32.release();
-    c->errflag.release();
+    if (c->err_h) cudaFreeHost(c->err_h);
+    if (c->res_h) cudaFreeHost(c->res_h);
     c->gwork.release();
     c->rwork.release();
     c->nlW.release();
@@ -2565,10 +2589,10 @@ extern "C" int lynx_gram_mixed(lynx_ctx* c, const float* Y, const float* HY, lon
     const GramPlan plan = gram_plan(rows, n);
     LYNX_TRY(c->gwork.ensure(plan.work_bytes));
     LYNX_TRY(c->info.ensure(3 * sizeof(int)));
-    if (!c->errflag.p) LYNX_TRY(ensure_zeroed(c, c->errflag, sizeof(int)));
+    LYNX_TRY(ensure_errflag(c));
     int* bad = c->info.as<int>() + 2;
     LYNX_CUDA_TRY(cudaMemsetAsync(bad, 0, sizeof(int), c->stream));
-    LYNX_TRY(launch_gram_i8(Y, HY, ld, rows, n, scale, plan, c->gwork.p, c->gwork.bytes, Ms, Hs, c->errflag.as<int>(),
+    LYNX_TRY(launch_gram_i8(Y, HY, ld, rows, n, scale, plan, c->gwork.p, c->gwork.bytes, Ms, Hs, c->err_d,
                             bad, c->stream));
     int h = 0;
     LYNX_CUDA_TRY(cudaMemcpyAsync(&h, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
@@ -2591,9 +2615,9 @@ extern "C" int lynx_rotate_mixed(lynx_ctx* c, const float* Y, long long ld, long
     LYNX_TRY(activate(c));
     const RotPlan rp = rot_plan(rows, n);
     LYNX_TRY(c->rwork.ensure(rp.work_bytes));
-    if (!c->errflag.p) LYNX_TRY(ensure_zeroed(c, c->errflag, sizeof(int)));
+    LYNX_TRY(ensure_errflag(c));
     LYNX_TRY(launch_colexp(Ms, n, c->rwork.p, rp, rows, c->stream));
-    LYNX_TRY(launch_rot_i8(Y, ld, rows, 1, 1, W, n, rp, c->rwork.p, c->rwork.bytes, psi, ldp, c->errflag.as<int>(),
+    LYNX_TRY(launch_rot_i8(Y, ld, rows, 1, 1, W, n, rp, c->rwork.p, c->rwork.bytes, psi, ldp, c->err_d,
                            c->stream));
     return check_errflag(c);
 }
@@ -2602,8 +2626,8 @@ extern "C" int lynx_selftest_wait_timeout(lynx_ctx* c, int spins) {
     LYNX_CHECK_ARG(c != nullptr, "null context");
     LYNX_CHECK_ARG(spins >= 1 && spins <= (1 << 20), "spins must lie in [1, 2^20]");
     LYNX_TRY(activate(c));
-    if (!c->errflag.p) LYNX_TRY(ensure_zeroed(c, c->errflag, sizeof(int)));
-    wait_selftest_kernel<<<1, 32, 0, c->stream>>>(spins, c->errflag.as<int>());
+    LYNX_TRY(ensure_errflag(c));
+    wait_selftest_kernel<<<1, 32, 0, c->stream>>>(spins, c->err_d);
     count_launch();
     LYNX_CUDA_TRY(cudaGetLastError());
     return check_errflag(c);

@@ -267,8 +267,25 @@ __global__ void __launch_bounds__(kEigThreads)
     nrm = 0.0;
     for (int w = 0; w < kEigThreads / 32; ++w) nrm += red[w];
     const double thr = 0x1p-54 * sqrt(nrm), inv = nrm > 0.0 ? rsqrt(nrm) : 0.0;
-    // Jacobi sweeps
+    // Jacobi sweeps.  A thread's tasks are the same in every round (2 x 2 blocks (P, Q) of A, then rows i of
+    // V and pairs Q): their indices are worked out once.
     const int np2 = NP / 2;
+    constexpr int NT = 3;  // N <= 40: 400 + 800 tasks
+    int ta[NT], tb[NT];    // (P, Q), or (-1 - i, Q), or (0, -1): nothing
+#pragma unroll
+    for (int k = 0; k < NT; ++k) {
+        const int w = tid + k * kEigThreads;
+        ta[k] = 0;
+        tb[k] = -1;
+        if (w < np2 * np2) {
+            ta[k] = w % np2;
+            tb[k] = w / np2;
+        } else if (w < np2 * np2 + np2 * N) {
+            const int f = w - np2 * np2;
+            ta[k] = -1 - f % N;
+            tb[k] = f / N;
+        }
+    }
     bool done = false;
     for (int sweep = 0; sweep < kMaxSweeps && !done; ++sweep) {
         // done when nothing is left to rotate
@@ -282,8 +299,10 @@ __global__ void __launch_bounds__(kEigThreads)
         for (int rnd = 0; rnd < NP - 1; ++rnd) {
             __syncthreads();
             if (tid < np2) {
-                int p = tid == 0 ? NP - 1 : (rnd + tid) % (NP - 1);
-                int q = tid == 0 ? rnd : (rnd + NP - 1 - tid) % (NP - 1);
+                int p = rnd + tid, q = rnd + NP - 1 - tid;  // round robin, modulo NP - 1
+                if (p >= NP - 1) p -= NP - 1;
+                if (q >= NP - 1) q -= NP - 1;
+                if (tid == 0) p = NP - 1;
                 if (p > q) {
                     const int s = p;
                     p = q;
@@ -306,9 +325,9 @@ __global__ void __launch_bounds__(kEigThreads)
                     if (m > thr) {
                         const float ms = (float)(m * inv), ds = (float)(d * inv);
                         const double t = 2.0f * ms / (ds + copysignf(sqrtf(fmaf(ds, ds, 4.0f * ms * ms)), ds));
-                        const double c2 = 1.0 / fma(t, t, 1.0);
                         c = rsqrt(fma(t, t, 1.0));
                         s = t * c;
+                        const double c2 = c * c;
                         dg[3 * tid] = fma(c2 * t, fma(t, d, -2.0 * m), app);
                         dg[3 * tid + 1] = fma(-c2 * t, fma(t, d, -2.0 * m), aqq);
                         dg[3 * tid + 2] = c2 * (m - t * fma(m, t, d));
@@ -324,9 +343,11 @@ __global__ void __launch_bounds__(kEigThreads)
             }
             __syncthreads();
             // columns p' = c p - s e* q, q' = s p + c e* q, rows by the conjugate
-            for (int w = tid; w < np2 * np2 + np2 * N; w += kEigThreads) {
-                if (w < np2 * np2) {
-                    const int P = w % np2, Q = w / np2;
+#pragma unroll
+            for (int k = 0; k < NT; ++k) {
+                if (tb[k] < 0) break;
+                if (ta[k] >= 0) {
+                    const int P = ta[k], Q = tb[k];
                     const int p1 = pq[2 * P], q1 = pq[2 * P + 1], p2 = pq[2 * Q], q2 = pq[2 * Q + 1];
                     const bool v1 = q1 < N, v2 = q2 < N;
                     const double c1 = cs[2 * P], s1 = v1 ? cs[2 * P + 1] : 0.0;
@@ -357,7 +378,7 @@ __global__ void __launch_bounds__(kEigThreads)
                     if (v1) A[q1 + p2 * N] = vadd(vscale(s1, b00), vscale(c1, r10));
                     if (v1 && v2) A[q1 + q2 * N] = vadd(vscale(s1, b01), vscale(c1, r11));
                 } else {
-                    const int f = w - np2 * np2, Q = f / N, i = f % N;
+                    const int Q = tb[k], i = -1 - ta[k];
                     const int p2 = pq[2 * Q], q2 = pq[2 * Q + 1];
                     const double c2 = cs[2 * Q], s2 = cs[2 * Q + 1];
                     if (q2 >= N || s2 == 0.0) continue;
