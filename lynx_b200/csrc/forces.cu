@@ -7,7 +7,7 @@
 // kinetic_kernel sums the six products of the gradients of all points as it marches through z.
 // One read of the orbitals each.  Forces and stress of Si64 (60^3, 160 states) together: 12.3 ms with a
 // gradient block written per direction (1.0 ms each), a gather of every block and three weighted copies
-// of the projectors made on the host on each call (about 4 ms); 2.3 ms here.
+// of the projectors made on the host on each call (about 4 ms); 2.0 ms here.
 #include <algorithm>
 #include <type_traits>
 
