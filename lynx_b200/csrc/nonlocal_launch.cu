@@ -114,7 +114,7 @@ int launch_nl_gather(const NLDev& nl, const T* x, long long ld, int ncol, T* alp
 template <typename T>
 int launch_nl_apply(const NLDev& nl, const T* x, long long ld, T* out, long long ldo, int ncol, double dV,
                     typename ScalarOf<T>::type scale, cudaStream_t st) {
-    if (nl.n_atom == 0 || ncol <= 0) return LYNX_OK;
+    if (nl.n_atom == 0 || nl.max_np == 0 || ncol <= 0) return LYNX_OK;
     if (!nl.compact || nl.max_np > 32) {
         set_error("the one-kernel nonlocal apply needs disjoint projector spheres and at most 32 projectors");
         return LYNX_ERR_UNSUPPORTED;

@@ -1,6 +1,8 @@
 """Kernels of small problems: the one-thread-per-point stencil, the one-kernel nonlocal apply of few
 atoms, and the four-launch Rayleigh-Ritz step of few states, against the numpy oracle, the pipelined
 stencil and dense linear algebra."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -70,6 +72,48 @@ def test_direct_step_is_the_pipelined_one(synth_psp8, precision, shape, ncol):
         ctx.set_option(_lib.OPT_STENCIL_SHAPE, forced)
         out.append(es.chebyshev_filter(x, V, 25.0, -2.0, 70.0, degree=5))
     assert np.array_equal(out[0], out[1])
+    ctx.close()
+
+
+def _drop_projectors(tab, atoms):
+    """The tables with the projectors of some atoms taken out; the atoms and their images stay."""
+    lens = tab.img_ndc * tab.atom_nproj[tab.img_atom]
+    keep = ~np.isin(tab.img_atom, atoms)
+    chi = np.concatenate([b for b, k in zip(np.split(tab.chi, np.cumsum(lens)[:-1]), keep) if k] or [np.zeros(0)])
+    nproj = tab.atom_nproj.copy()
+    nproj[atoms] = 0
+    gamma = np.concatenate([g for a, g in enumerate(np.split(tab.gamma, np.cumsum(tab.atom_nproj)[:-1]))
+                            if a not in atoms] or [np.zeros(0)])
+    return dataclasses.replace(tab, atom_nproj=nproj, chi=chi, gamma=gamma)
+
+
+@pytest.mark.parametrize("kpt", [False, True])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_atoms_without_projectors(synth_psp8, precision, kpt):
+    """A filter with tables in which no atom has projectors is the filter without tables, bitwise; with
+    every other atom left, H psi is the oracle's (1e-12 as above)."""
+    from lynx_b200 import solver
+    cl, pos, V = _cell("si8", (20, 21, 22))
+    tab = P.nonlocal_tables(cl, pos, P.read_psp8(synth_psp8))
+    ctx = solver.Context(cl)
+    k = np.array([0.25, -0.125, 0.375]) * 2 * np.pi / cl.lengths
+    ctx.set_kpoint(k)
+    es = solver.EigenSolver(ctx, precision)
+    x = C.random_orbitals(ctx.nd, 5, seed=4, complex_=kpt)
+    out = []
+    for t in (None, _drop_projectors(tab, np.arange(tab.n_atom))):
+        ctx.set_nonlocal(t)
+        out.append(es.chebyshev_filter(x, V, 25.0, -2.0, 70.0, degree=9, kpt=kpt))
+    assert np.array_equal(out[0], out[1])
+    drop = np.arange(0, tab.n_atom, 2)
+    ctx.set_nonlocal(_drop_projectors(tab, drop))
+    h = solver.Hamiltonian(ctx, V)
+    gamma = tab.gamma.reshape(tab.n_atom, -1).copy()
+    gamma[drop] = 0.0  # the oracle takes one projector count: no strength instead of no projector
+    zero = dataclasses.replace(tab, gamma=gamma.ravel())
+    want = _oracle(cl, zero).apply(x, V, kpt=k if kpt else None)
+    got = h.apply_kpt(x) if kpt else h.apply(x)
+    assert np.abs(got - want).max() < 1e-12 * np.abs(want).max()
     ctx.close()
 
 

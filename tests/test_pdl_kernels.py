@@ -1,0 +1,40 @@
+"""Kernels of programmatic dependent launches: every thread waits for the grid before it, whatever it has
+to do.  Read off the sources (no GPU): what a kernel does not wait for depends on timing."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "lynx_b200", "csrc")
+
+
+def _kernels():
+    """(name, parameters, body) of every kernel that calls pdl_wait(), comments taken out."""
+    out = []
+    for f in sorted(os.listdir(CSRC)):
+        if not f.endswith((".cu", ".cuh")):
+            continue
+        with open(os.path.join(CSRC, f)) as fh:
+            src = re.sub(r"//[^\n]*", "", fh.read())
+        for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\([^;{]*?\)\)?\s*)?(\w+)\s*\(([^;{]*?)\)\s*\{", src):
+            depth, i = 1, m.end()
+            while depth:
+                depth += {"{": 1, "}": -1}.get(src[i], 0)
+                i += 1
+            if "pdl_wait();" in src[m.end():i]:
+                out.append((m.group(1), m.group(2), src[m.end():i]))
+    return out
+
+
+KERNELS = _kernels()
+
+
+def test_the_kernels_are_found():
+    assert {k[0] for k in KERNELS} >= {"direct_step_kernel", "nonorth_mixed_kernel", "nl_atom_kernel"}
+
+
+@pytest.mark.parametrize("name,params,body", KERNELS, ids=[k[0] for k in KERNELS])
+def test_no_return_before_the_wait(name, params, body):
+    waits = [m.start() for m in re.finditer(r"pdl_wait\(\);", body)]
+    for m in re.finditer(r"\breturn;", body):
+        assert waits[0] < m.start(), f"{name} leaves before pdl_wait()"
