@@ -12,6 +12,9 @@
  *     std::complex<double>.
  *   - Operator entry points take DEVICE pointers and run on the context's
  *     stream (lynx_set_stream).  The *_host entry points take host pointers.
+ *     A call's work is complete when it returns; only lynx_nonlocal_apply,
+ *     _kpt and _noalloc, lynx_pair_density and lynx_randomize_orbitals return
+ *     with work in flight on the stream.
  *   - Every call returns LYNX_OK or an error status; lynx_last_error() gives
  *     the message of the last failing call on the calling thread.  Nothing
  *     calls exit(): a CUDA or solver failure is reported, not fatal.

@@ -740,9 +740,19 @@ int ensure_errflag(lynx_ctx* c) {
     return LYNX_OK;
 }
 
+// The end of a call: waits for its work and reports a bounded wait that gave up.  It waits whichever
+// kernels ran, not only where there is a flag to look at: the blocks, row layouts and projections that
+// the work uses are the context's, and the next call may come on another stream.  Recorded work (stream
+// capture) has nothing to wait for; kernels with bounded waits are not recorded, as their flag could not
+// be looked at.
 int check_errflag(lynx_ctx* c) {
-    if (!c->err_h) return LYNX_OK;
+    if (!c->err_h) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        LYNX_CUDA_TRY(cudaStreamIsCapturing(c->stream, &cap));
+        if (cap != cudaStreamCaptureStatusNone) return LYNX_OK;
+    }
     LYNX_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    if (!c->err_h) return LYNX_OK;
     volatile int* flag = c->err_h;
     if (*flag) {
         *flag = 0;
