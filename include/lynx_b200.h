@@ -78,7 +78,8 @@ LYNX_API int lynx_create(lynx_ctx** out, int device, int nx, int ny, int nz, int
                 int orthogonal, const int* bc);
 LYNX_API int lynx_destroy(lynx_ctx* ctx);
 
-/* CUDA stream (cudaStream_t) for all later work on this context; NULL = the legacy default stream. */
+/* CUDA stream (cudaStream_t) for all later work on this context; NULL = the legacy default stream.
+ * The new stream waits for work that an earlier call left in flight on the context's own memory. */
 LYNX_API int lynx_set_stream(lynx_ctx* ctx, void* stream);
 
 /* Nd, dV (FDGrid::dV, src/core/FDGrid.cpp:33) and the largest eigenvalue of -0.5*Lap

@@ -336,6 +336,10 @@ struct lynx_ctx {
     int* err_d = nullptr;
     double* res_h = nullptr;
     size_t res_n = 0;
+    // Marks the work on `alpha` that a call left in flight (leave_in_flight): lynx_set_stream makes
+    // another stream wait for it.
+    cudaEvent_t in_flight = nullptr;
+    bool pending = false;
     DevBuf gwork;           // slices, exponents and split partials of the tensor-core Gram
     DevBuf rwork;           // slices and exponents of the tensor-core rotation
     DevBuf cplx_work;       // planar split and real 2N x 2N products of the mixed k-point Rayleigh-Ritz
@@ -752,6 +756,7 @@ int check_errflag(lynx_ctx* c) {
         if (cap != cudaStreamCaptureStatusNone) return LYNX_OK;
     }
     LYNX_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    c->pending = false;
     if (!c->err_h) return LYNX_OK;
     volatile int* flag = c->err_h;
     if (*flag) {
@@ -759,6 +764,17 @@ int check_errflag(lynx_ctx* c) {
         set_error("a bounded device-side wait gave up (shared-memory pipeline did not complete)");
         return LYNX_ERR_TIMEOUT;
     }
+    return LYNX_OK;
+}
+
+// The end of a call that returns with work in flight on the context's projections.
+int leave_in_flight(lynx_ctx* c) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    LYNX_CUDA_TRY(cudaStreamIsCapturing(c->stream, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return LYNX_OK;
+    if (!c->in_flight) LYNX_CUDA_TRY(cudaEventCreateWithFlags(&c->in_flight, cudaEventDisableTiming));
+    LYNX_CUDA_TRY(cudaEventRecord(c->in_flight, c->stream));
+    c->pending = true;
     return LYNX_OK;
 }
 
@@ -1762,6 +1778,7 @@ int lynx_destroy(lynx_ctx* c) {
     c->vpad32.release();
     if (c->err_h) cudaFreeHost(c->err_h);
     if (c->res_h) cudaFreeHost(c->res_h);
+    if (c->in_flight) cudaEventDestroy(c->in_flight);
     c->gwork.release();
     c->rwork.release();
     c->nlW.release();
@@ -1794,7 +1811,15 @@ int lynx_destroy(lynx_ctx* c) {
 
 int lynx_set_stream(lynx_ctx* c, void* stream) {
     LYNX_CHECK_ARG(c != nullptr, "null context");
-    c->stream = static_cast<cudaStream_t>(stream);
+    const cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (c->pending && s != c->stream) {
+        LYNX_CUDA_TRY(cudaSetDevice(c->device));
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        LYNX_CUDA_TRY(cudaStreamIsCapturing(s, &cap));
+        // (recorded work is ordered by whoever replays it)
+        if (cap == cudaStreamCaptureStatusNone) LYNX_CUDA_TRY(cudaStreamWaitEvent(s, c->in_flight, 0));
+    }
+    c->stream = s;
     return LYNX_OK;
 }
 
@@ -2091,7 +2116,8 @@ int lynx_nonlocal_apply(lynx_ctx* c, const double* psi, double* hpsi, int ncol, 
     const int ncolp = ((ncol + kNLColBlock - 1) / kNLColBlock) * kNLColBlock;
     LYNX_TRY(c->alpha.ensure(sizeof(double) * (size_t)c->nl.total_proj * ncolp));
     LYNX_TRY(launch_nl_gather<double>(c->nl, psi, l, ncol, c->alpha.as<double>(), ncolp, c->dV, c->stream));
-    return launch_nl_scatter<double, double>(c->nl, hpsi, l, ncol, c->alpha.as<double>(), ncolp, 1.0, c->stream);
+    LYNX_TRY(launch_nl_scatter<double, double>(c->nl, hpsi, l, ncol, c->alpha.as<double>(), ncolp, 1.0, c->stream));
+    return leave_in_flight(c);
 }
 
 int lynx_nonlocal_apply_kpt(lynx_ctx* c, const double* psi, double* hpsi, int ncol, int ld) {
@@ -2105,8 +2131,9 @@ int lynx_nonlocal_apply_kpt(lynx_ctx* c, const double* psi, double* hpsi, int nc
     LYNX_TRY(c->alpha.ensure(sizeof(double2) * (size_t)c->nl.total_proj * ncolp));
     LYNX_TRY(launch_nl_gather<double2>(c->nl, reinterpret_cast<const double2*>(psi), l, ncol,
                                        c->alpha.as<double2>(), ncolp, c->dV, c->stream));
-    return launch_nl_scatter<double2, double>(c->nl, reinterpret_cast<double2*>(hpsi), l, ncol,
-                                              c->alpha.as<double2>(), ncolp, 1.0, c->stream);
+    LYNX_TRY(launch_nl_scatter<double2, double>(c->nl, reinterpret_cast<double2*>(hpsi), l, ncol,
+                                                c->alpha.as<double2>(), ncolp, 1.0, c->stream));
+    return leave_in_flight(c);
 }
 
 static int filter_entry(lynx_ctx* c, const double* X, double* Y, const double* veff, int ncol, int ld, double lc,

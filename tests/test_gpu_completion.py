@@ -78,3 +78,29 @@ def test_recorded_call_replays(si8):
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize("kpt", [False, True])
+def test_nonlocal_apply_on_another_stream_waits(si8, kpt):
+    """The nonlocal apply returns with its work in flight; one on another stream, which uses the same
+    projections of the context, waits for it."""
+    import time
+    import torch
+    from lynx_b200 import solver
+    cl, V, ctx = si8
+    nl = solver.NonlocalProjector(ctx)
+    xs = [_block(ctx, 5, 3 + i, kpt) for i in range(2)]
+    want = [nl.apply(x, torch.zeros_like(x), kpt=kpt).clone() for x in xs]
+    got = [torch.zeros_like(x) for x in xs]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in xs]
+    with torch.cuda.stream(streams[0]):
+        torch.cuda._sleep(20 * LONG)
+        nl.apply(xs[0], got[0], kpt=kpt)
+    with torch.cuda.stream(streams[1]):
+        nl.apply(xs[1], got[1], kpt=kpt)
+    time.sleep(0.05)
+    assert not streams[0].query() and not streams[1].query()
+    torch.cuda.synchronize()
+    for g, w in zip(got, want):
+        assert torch.equal(g, w)
