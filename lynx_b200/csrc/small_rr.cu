@@ -421,15 +421,16 @@ __global__ void __launch_bounds__(kEigThreads)
 }
 
 // psi(:, j) = sum_i Y(:, i) W(i, j), FP64 sums in the order of i; thread = one grid point x
-// kRotCols columns.
+// kRotCols columns.  psi stays as it is where the subspace algebra failed (info): W is not there then.
 constexpr int kRotCols = 8;
 template <typename T>
 __global__ void __launch_bounds__(128)
     small_rotate_kernel(const T* __restrict__ Y, long long ld, int nx, int nxp, long long nd, int N,
-                        const typename Wide<T>::type* __restrict__ W, typename Wide<T>::type* __restrict__ psi,
-                        long long ldp) {
+                        const typename Wide<T>::type* __restrict__ W, const int* __restrict__ info,
+                        typename Wide<T>::type* __restrict__ psi, long long ldp) {
     using D = typename Wide<T>::type;
     __shared__ D ws[kSmallRRMax * kRotCols];
+    if (info[0] | info[1] | info[2]) return;
     const int j0 = blockIdx.y * kRotCols;
     for (int e = threadIdx.x; e < N * kRotCols; e += 128) {
         const int i = e / kRotCols, j = j0 + e % kRotCols;
@@ -481,7 +482,7 @@ int launch_small_rr(const T* Y, const T* HY, long long ld, long long rows, int n
     LYNX_CUDA_TRY(smem_cap(small_eig_kernel<W>, se));
     small_eig_kernel<W><<<1, kEigThreads, se, st>>>(ms, hs, n, eig, info);
     dim3 grid((unsigned)((nd + 127) / 128), (n + kRotCols - 1) / kRotCols);
-    small_rotate_kernel<T><<<grid, 128, 0, st>>>(Y, ld, nx, nxp, nd, n, hs, static_cast<W*>(psi), ldp);
+    small_rotate_kernel<T><<<grid, 128, 0, st>>>(Y, ld, nx, nxp, nd, n, hs, info, static_cast<W*>(psi), ldp);
     count_launch(4);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {

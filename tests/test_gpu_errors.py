@@ -53,6 +53,32 @@ def test_rank_deficient_start_block_is_chol_fail(sys8, prec):
     assert ei.value.status == _lib.LYNX_ERR_CHOL_FAIL
 
 
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("density", [False, True])
+@pytest.mark.parametrize("fault", ["nan", "rank"])
+def test_failed_pass_of_few_states_leaves_the_orbitals(sys8, prec, density, fault):
+    """Up to 40 states the rotation is launched before the host knows of the failure: it must not run."""
+    import torch
+    s = sys8
+    psi = C.random_orbitals(s["ctx"].nd, 8, seed=6)
+    V = s["V"].copy()
+    if fault == "nan":
+        V[1234] = np.nan
+    else:
+        psi[:, 3] = 0.0
+    t = torch.from_numpy(np.ascontiguousarray(psi.T)).cuda()
+    before = t.clone()
+    es = s["solver"].EigenSolver(s["ctx"], prec)
+    lc = 0.5 * (s["lo"] + s["hi"])
+    with pytest.raises(_lib.LynxError) as ei:
+        if density:
+            es.solve_density(t, V, lc, s["lo"], s["hi"], 6, nelectron=4.0)
+        else:
+            es.solve(t, V, lc, s["lo"], s["hi"], 6)
+    assert ei.value.status == (_lib.LYNX_ERR_NONFINITE if fault == "nan" else _lib.LYNX_ERR_CHOL_FAIL)
+    assert torch.equal(t, before)
+
+
 def test_bounded_wait_times_out_and_context_recovers(sys8):
     s = sys8
     ctx = s["ctx"]
