@@ -64,6 +64,8 @@ __device__ __forceinline__ double mod_phase(double2 a, double2& e) {
 }
 __device__ __forceinline__ bool fin(double a) { return isfinite(a); }
 __device__ __forceinline__ bool fin(double2 a) { return isfinite(a.x) && isfinite(a.y); }
+__device__ __forceinline__ double amax(double a) { return fabs(a); }
+__device__ __forceinline__ double amax(double2 a) { return fmax(fabs(a.x), fabs(a.y)); }
 __device__ __forceinline__ void set_re(double& a, double v) { a = v; }
 __device__ __forceinline__ void set_re(double2& a, double v) { a = make_double2(v, 0.0); }
 __device__ __forceinline__ double sub(double a, double b) { return a - b; }
@@ -184,6 +186,7 @@ __global__ void __launch_bounds__(kEigThreads)
     double* red = dg + NP + NP / 2;                            // [kEigThreads / 32]
     int* pq = reinterpret_cast<int*>(red + kEigThreads / 32);  // [NP/2][2] rows of the pair (p < 0: idle)
     int* rank = pq + NP;                              // [N]
+    __shared__ double big[kEigThreads / 32];
     __shared__ int bad, chol, moved;
     if (tid == 0) bad = chol = 0;
     __syncthreads();
@@ -249,23 +252,54 @@ __global__ void __launch_bounds__(kEigThreads)
         }
         __syncthreads();
     }
-    double nrm = 0.0;
+    // symmetric part, its norm and its largest entry
+    double nrm = 0.0, top = 0.0;
     for (int e = tid; e < n2; e += kEigThreads) {
         const int i = e % N, j = e / N;
         if (i > j) continue;
         const W h = vscale(0.5, vadd(A[e], cj(A[j + i * N])));
+        if (!fin(h)) bad = 1;
         A[e] = h;
         A[j + i * N] = cj(h);
         if (i == j) set_re(A[e], re(h));
         const double v = mod(h);
         nrm = fma(v, i == j ? v : 2.0 * v, nrm);
+        top = fmax(top, amax(h));
     }
+    auto sum_all = [&](double v) {  // over the CTA, in a fixed order
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
-    if ((tid & 31) == 0) red[tid >> 5] = nrm;
-    __syncthreads();
-    nrm = 0.0;
-    for (int w = 0; w < kEigThreads / 32; ++w) nrm += red[w];
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if ((tid & 31) == 0) red[tid >> 5] = v;
+        __syncthreads();
+        v = 0.0;
+        for (int w = 0; w < kEigThreads / 32; ++w) v += red[w];
+        return v;
+    };
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+    if ((tid & 31) == 0) big[tid >> 5] = top;
+    nrm = sum_all(nrm);
+    top = 0.0;
+    for (int w = 0; w < kEigThreads / 32; ++w) top = fmax(top, big[w]);
+    if (bad) {
+        if (tid == 0) info[2] = 1;
+        return;
+    }
+    // Entries whose squares leave the range of FP64 are scaled by a power of two, and the eigenvalues back.
+    double up = 1.0;
+    if (top > 0.0 && (top > 0x1p+400 || top < 0x1p-400)) {
+        const int k = max(-1000, min(1000, ilogb(top)));
+        up = ldexp(1.0, k);
+        const double dn = ldexp(1.0, -k);
+        double s = 0.0;
+        __syncthreads();  // red is summed up again
+        for (int e = tid; e < n2; e += kEigThreads) {
+            A[e] = vscale(dn, A[e]);
+            const double v = mod(A[e]);
+            s = fma(v, v, s);
+        }
+        nrm = sum_all(s);
+    }
     const double thr = 0x1p-54 * sqrt(nrm), inv = nrm > 0.0 ? rsqrt(nrm) : 0.0;
     // Jacobi sweeps.  A thread's tasks are the same in every round (2 x 2 blocks (P, Q) of A, then rows i of
     // V and pairs Q): their indices are worked out once.
@@ -403,7 +437,7 @@ __global__ void __launch_bounds__(kEigThreads)
             r += (u < v || (u == v && j < i)) ? 1 : 0;
         }
         rank[i] = r;
-        eig[r] = v;
+        eig[r] = up * v;
     }
     // V <- L^-H V
     for (int k = N - 1; k >= 0; --k) {

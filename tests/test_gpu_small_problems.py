@@ -163,3 +163,26 @@ def test_degenerate_states(n):
     assert np.abs(eig - np.array([0.0] + [e1] * (n - 1))).max() < 1e-11
     assert np.abs(psi.T @ psi * cl.dV - np.eye(n)).max() < 1e-11
     ctx.close()
+
+
+@pytest.mark.parametrize("kpt", [False, True])
+@pytest.mark.parametrize("n", [5, 24])
+def test_ritz_values_far_from_one(n, kpt):
+    """H of size 2^-590 or 2^560, whose entries' squares leave the range of FP64.  A cell 2^300 times as
+    wide is exactly 2^-600 of the same H; a potential of 2^560 against one of 2^100 leaves the kinetic term
+    below rounding, so the values differ by 2^460 to the rounding of the products (about 1e3 terms)."""
+    from lynx_b200 import solver
+    cl = C.diamond_si(1, (15, 14, 16))[0]
+    x = C.random_orbitals(cl.nd, n, seed=8, complex_=kpt)
+    v = np.random.default_rng(3).normal(size=cl.nd)
+
+    def ritz(scale, V, s):
+        ctx = solver.Context(C.Cell(cl.latvec * scale, cl.shape))
+        es = solver.EigenSolver(ctx, "fp64")
+        _, eig = (es.solve_kpt if kpt else es.solve)(x, V, 25.0 * s, -9.0 * s, 70.0 * s, 1)
+        ctx.close()
+        return eig
+
+    assert np.array_equal(ritz(2.0 ** 300, v * 2.0 ** -600, 2.0 ** -600), ritz(1.0, v, 1.0) * 2.0 ** -600)
+    a, b = (ritz(1.0, v * 2.0 ** e, 2.0 ** e) for e in (100, 560))
+    assert np.abs(b * 2.0 ** -460 - a).max() < 1e-12 * np.abs(a).max()
