@@ -44,6 +44,16 @@ def _torch():
     return torch
 
 
+def _has_memory(t) -> bool:
+    """Whether a tensor's values lie in memory of its own: not those of a batched tensor (a backward under
+    vmap, is_grads_batched) or of a view that is negated when it is read."""
+    try:
+        t.data_ptr()
+    except RuntimeError:
+        return False
+    return not t.is_neg()
+
+
 def _make_fns():
     torch = _torch()
     from . import solver
@@ -67,10 +77,12 @@ def _make_fns():
             grad_psi = solver.Hamiltonian(fctx.ctx).apply(g, Veff=veff.contiguous()) if fctx.needs_input_grad[0] else None
             grad_v = None
             if fctx.needs_input_grad[1]:
-                # one kernel, unless this backward is itself recorded (create_graph) or the block is one
-                # vector: then torch's own operations
-                plain = not torch.is_grad_enabled() and psi.dim() == 2 and psi.dtype == torch.float64 and psi.is_cuda
-                grad_v = solver.pair_density(fctx.ctx, g, psi.contiguous()) if plain else (g * psi).sum(0)
+                # one kernel, unless this backward is itself recorded (create_graph), the block is one vector
+                # or a tensor is not plain memory: then torch's own operations
+                p = psi.contiguous()
+                plain = (not torch.is_grad_enabled() and psi.dim() == 2 and psi.dtype == torch.float64 and psi.is_cuda
+                         and _has_memory(g) and _has_memory(p))
+                grad_v = solver.pair_density(fctx.ctx, g, p) if plain else (g * psi).sum(0)
             grad_pos = None
             if fctx.needs_input_grad[2]:
                 ones = np.ones(psi.shape[0])
