@@ -253,11 +253,22 @@ constexpr int kExpTilePts = 512;
 
 template <typename T>
 int launch_nl_gather(const NLDev& nl, const T* x, long long ld, int ncol, T* alpha, int ncolp, double dV,
-                     cudaStream_t st);
-// Few atoms: a gather by (atom, 64 columns) leaves most SMs idle, and one kernel can take an atom's
-// gather and its term together.
+                     cudaStream_t st, bool few);
+// Few atoms and columns: a gather by (atom, 64 columns) leaves most SMs idle, and one kernel can take an
+// atom's gather and its term together, one CTA per 2 or 4 columns.  Every CTA reads the atom's projector
+// values again, so with many (atom, column) pairs the staged gather and the term fused into the stencil
+// are the better ones.  Us a degree, FP32 / FP64, this kernel against those: 8 atoms (30^3), 256 columns
+// 84 / 128 against 105 / 144, 520 columns 163 / 238 against 146 / 223; 16 atoms, 128 columns 88 / 130
+// against 111 / 139, 256 columns 161 / 244 against 144 / 215; 24 atoms, 64 columns 62 / 106 against 91 / 130, 256
+// columns 246 / 337 against 191 / 282.  Complex data have the atom kernel's gather in any case, and here
+// save the scatter.  cols: the columns of the caller's whole block, also where it is filtered in column
+// blocks (the two gathers add in different orders).
 constexpr int kNLFewAtoms = 32;
-bool nl_few_atoms(const NLDev& nl);
+constexpr long long kNLFewPairs = 2048;  // real data: atoms x columns
+template <typename T>
+bool nl_few_atoms(const NLDev& nl, int cols) {
+    return nl.n_atom < kNLFewAtoms && (ScalarOf<T>::cplx || (long long)nl.n_atom * cols <= kNLFewPairs);
+}
 // out += scale * chi Gamma dV chi^T x in one kernel (disjoint spheres: nl.compact, at most 32
 // projectors per atom); bitwise launch_nl_gather + launch_nl_scatter for few atoms and complex data.
 template <typename T>

@@ -366,6 +366,7 @@ struct lynx_ctx {
     // first column of every column block with the event that marks its arrival on the device.
     cudaStream_t copy_stream = nullptr;
     std::vector<std::pair<int, cudaEvent_t>> col_blocks;
+    int col_total = 0;  // columns of all blocks together
     // nonlocal tables re-indexed for padded row layouts: nxp -> tables
     std::map<int, NLDev> nl_layouts;
     std::vector<DevBuf> nl_layout_bufs;
@@ -866,6 +867,9 @@ template <typename T> bool direct_step_pays(long long nd, int ncol) {
     return ScalarOf<T>::cplx || nd * ncol * (long long)sizeof(T) <= kDirectRealBytes;
 }
 
+// Columns of the block that a step's ncol columns belong to.
+int whole_cols(const lynx_ctx* c, int ncol) { return c->col_total > 0 ? c->col_total : ncol; }
+
 // One Chebyshev step out = a H x + b x + d xold (H with the nonlocal term when tables are set).
 // With the fused nonlocal path, xs_in (optional) is the compact sphere-point copy of x written
 // by the previous step, and xs_out (optional) receives the compact copy of out; *xs_written
@@ -890,7 +894,8 @@ int cheb_step(lynx_ctx* c, int nxp, const T* x, long long ldx, const T* xold, lo
     // values (chi alpha) are expanded to the compact point numbering and added by the stencil
     // kernel itself (out += a * W), in the order the separate scatter would add them.
     // Few atoms: one kernel after the stencil does the gather and the term together.
-    const bool few = c->has_nl && c->nl.compact && c->nl.max_np <= 32 && nl_few_atoms(c->nl);
+    const bool few_pairs = nl_few_atoms<T>(c->nl, whole_cols(c, ncol));
+    const bool few = c->has_nl && c->nl.compact && c->nl.max_np <= 32 && few_pairs;
     const bool fuse = c->has_nl && !few && c->fuse_nl && c->orth && pipe_ok && !ScalarOf<T>::cplx && !use_k && c->nl.compact &&
                       c->nl.n_colors == 1 && geom(c).R == 6 && c->bc[0] == LYNX_BC_PERIODIC &&
                       c->bc[1] == LYNX_BC_PERIODIC && c->bc[2] == LYNX_BC_PERIODIC;
@@ -905,9 +910,9 @@ int cheb_step(lynx_ctx* c, int nxp, const T* x, long long ldx, const T* xold, lo
             // gather from the dense compact copy: entries index it through ent_pt
             NLDev cv = *nl;
             cv.gpos = c->nl.ent_pt;
-            LYNX_TRY(launch_nl_gather<T>(cv, xs_in, ldw, ncol, c->alpha.as<T>(), ncolp, c->dV, c->stream));
+            LYNX_TRY(launch_nl_gather<T>(cv, xs_in, ldw, ncol, c->alpha.as<T>(), ncolp, c->dV, c->stream, few_pairs));
         } else {
-            LYNX_TRY(launch_nl_gather<T>(*nl, x, ldx, ncol, c->alpha.as<T>(), ncolp, c->dV, c->stream));
+            LYNX_TRY(launch_nl_gather<T>(*nl, x, ldx, ncol, c->alpha.as<T>(), ncolp, c->dV, c->stream, few_pairs));
         }
     }
     const long long ldg = (long long)nxp * c->ny * c->nz;
@@ -968,7 +973,7 @@ template <typename T>
 int compact_bufs(lynx_ctx* c, int ncol, T* xs[2]) {
     xs[0] = xs[1] = nullptr;
     if (ScalarOf<T>::cplx || !c->has_nl || !c->fuse_nl || !c->fuse_compact_gather || !c->nl.compact ||
-        c->nl.n_colors != 1 || nl_few_atoms(c->nl))
+        c->nl.n_colors != 1 || nl_few_atoms<T>(c->nl, whole_cols(c, ncol)))
         return LYNX_OK;
     const long long ldw = ((long long)c->nl.n_pts + 3) & ~3LL;
     for (int i = 0; i < 2; ++i) {
@@ -2115,7 +2120,8 @@ int lynx_nonlocal_apply(lynx_ctx* c, const double* psi, double* hpsi, int ncol, 
     LYNX_TRY(activate(c));
     const int ncolp = ((ncol + kNLColBlock - 1) / kNLColBlock) * kNLColBlock;
     LYNX_TRY(c->alpha.ensure(sizeof(double) * (size_t)c->nl.total_proj * ncolp));
-    LYNX_TRY(launch_nl_gather<double>(c->nl, psi, l, ncol, c->alpha.as<double>(), ncolp, c->dV, c->stream));
+    LYNX_TRY(launch_nl_gather<double>(c->nl, psi, l, ncol, c->alpha.as<double>(), ncolp, c->dV, c->stream,
+                                      nl_few_atoms<double>(c->nl, ncol)));
     LYNX_TRY(launch_nl_scatter<double, double>(c->nl, hpsi, l, ncol, c->alpha.as<double>(), ncolp, 1.0, c->stream));
     return leave_in_flight(c);
 }
@@ -2130,7 +2136,8 @@ int lynx_nonlocal_apply_kpt(lynx_ctx* c, const double* psi, double* hpsi, int nc
     const int ncolp = ((ncol + kNLColBlock - 1) / kNLColBlock) * kNLColBlock;
     LYNX_TRY(c->alpha.ensure(sizeof(double2) * (size_t)c->nl.total_proj * ncolp));
     LYNX_TRY(launch_nl_gather<double2>(c->nl, reinterpret_cast<const double2*>(psi), l, ncol,
-                                       c->alpha.as<double2>(), ncolp, c->dV, c->stream));
+                                       c->alpha.as<double2>(), ncolp, c->dV, c->stream,
+                                       nl_few_atoms<double2>(c->nl, ncol)));
     LYNX_TRY(launch_nl_scatter<double2, double>(c->nl, reinterpret_cast<double2*>(hpsi), l, ncol,
                                                 c->alpha.as<double2>(), ncolp, 1.0, c->stream));
     return leave_in_flight(c);
@@ -2236,9 +2243,11 @@ int lynx_eigensolver_solve_host(lynx_ctx* c, double* psi, double* eig, const dou
     } else {
         LYNX_CUDA_TRY(cudaMemcpy2DAsync(dpsi.p, Nd * 8, psi, l * 8, Nd * 8, nband, cudaMemcpyHostToDevice, c->stream));
     }
+    c->col_total = pipelined ? nband : 0;
     int st = lynx_eigensolver_solve(c, dpsi.as<double>(), eig, dv.as<double>(), nband, (int)Nd, lc, emin, emax,
                                     degree, precision, lc_out);
     c->col_blocks.clear();
+    c->col_total = 0;
     if (pipelined) {
         cudaStreamSynchronize(c->copy_stream);
         for (cudaEvent_t e : evs) cudaEventDestroy(e);
@@ -3049,6 +3058,7 @@ extern "C" int lynx_nonlocal_apply_noalloc(lynx_ctx* c, const double* psi, doubl
     void* scratch = nullptr;
     LYNX_TRY(noalloc_scratch(c->device, &scratch));
     double* alpha = static_cast<double*>(scratch);
-    LYNX_TRY(launch_nl_gather<double>(c->nl, psi, l, ncol, alpha, ncolp, c->dV, c->stream));
+    LYNX_TRY(launch_nl_gather<double>(c->nl, psi, l, ncol, alpha, ncolp, c->dV, c->stream,
+                                      nl_few_atoms<double>(c->nl, ncol)));
     return launch_nl_scatter<double, double>(c->nl, hpsi, l, ncol, alpha, ncolp, 1.0, c->stream);
 }

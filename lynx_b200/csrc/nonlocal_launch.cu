@@ -95,18 +95,16 @@ int launch_atom_kernel(const NLDev& nl, const T* x, long long ld, int ncol, T* a
 }
 }  // namespace
 
-bool nl_few_atoms(const NLDev& nl) { return nl.n_atom < kNLFewAtoms; }
-
 template <typename T>
 int launch_nl_gather(const NLDev& nl, const T* x, long long ld, int ncol, T* alpha, int ncolp, double dV,
-                     cudaStream_t st) {
+                     cudaStream_t st, bool few) {
     if (nl.n_atom == 0 || ncol <= 0) return LYNX_OK;
     if (nl.max_np > 32) {
         set_error("%d projectors per atom exceed the gather kernel's limit of 32", nl.max_np);
         return LYNX_ERR_UNSUPPORTED;
     }
     if constexpr (kReal<T>) {
-        if (!nl_few_atoms(nl)) return gather2_dispatch<T>(nl, x, ld, ncol, alpha, ncolp, dV, st);
+        if (!few) return gather2_dispatch<T>(nl, x, ld, ncol, alpha, ncolp, dV, st);
     }
     return launch_atom_kernel<T, false>(nl, x, ld, ncol, alpha, ncolp, dV, nullptr, 0, 0, st);
 }
@@ -218,10 +216,10 @@ int launch_nl_expand(const NLDev& nl, T* W, long long ldw, int ncol, const T* al
 
 template int launch_nl_expand<double>(const NLDev&, double*, long long, int, const double*, int, cudaStream_t);
 template int launch_nl_expand<float>(const NLDev&, float*, long long, int, const float*, int, cudaStream_t);
-template int launch_nl_gather<double>(const NLDev&, const double*, long long, int, double*, int, double, cudaStream_t);
-template int launch_nl_gather<float>(const NLDev&, const float*, long long, int, float*, int, double, cudaStream_t);
-template int launch_nl_gather<double2>(const NLDev&, const double2*, long long, int, double2*, int, double, cudaStream_t);
-template int launch_nl_gather<float2>(const NLDev&, const float2*, long long, int, float2*, int, double, cudaStream_t);
+template int launch_nl_gather<double>(const NLDev&, const double*, long long, int, double*, int, double, cudaStream_t, bool);
+template int launch_nl_gather<float>(const NLDev&, const float*, long long, int, float*, int, double, cudaStream_t, bool);
+template int launch_nl_gather<double2>(const NLDev&, const double2*, long long, int, double2*, int, double, cudaStream_t, bool);
+template int launch_nl_gather<float2>(const NLDev&, const float2*, long long, int, float2*, int, double, cudaStream_t, bool);
 template int launch_nl_scatter<double, double>(const NLDev&, double*, long long, int, const double*, int, double, cudaStream_t);
 template int launch_nl_scatter<float, float>(const NLDev&, float*, long long, int, const float*, int, float, cudaStream_t);
 template int launch_nl_scatter<double2, double>(const NLDev&, double2*, long long, int, const double2*, int, double, cudaStream_t);

@@ -56,6 +56,57 @@ def test_h_apply_of_small_blocks(synth_psp8, kind, shape, ncol, kpt, fd_order):
     ctx.close()
 
 
+def _launches(ctx, f):
+    ctx.lib.lynx_launch_count(1)
+    out = f()
+    return out, ctx.lib.lynx_launch_count(0)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_atom_kernel_up_to_2048_pairs(synth_psp8, precision):
+    """8 atoms: 256 columns take the one-kernel apply (two launches a degree), 257 the staged gather, the
+    expansion and the fused term (three).  The same sums in another order: the columns agree to 100
+    roundings of the largest value (2^-53, 2^-24), a degree-3 filter's growth included."""
+    from lynx_b200 import solver
+    cl, pos, V = _cell("si8", (20, 18, 20))
+    ctx = solver.Context(cl)
+    ctx.set_option(_lib.OPT_AUTOTUNE, 0)
+    ctx.set_nonlocal(P.nonlocal_tables(cl, pos, P.read_psp8(synth_psp8)))
+    es = solver.EigenSolver(ctx, precision)
+    x = C.random_orbitals(ctx.nd, 257, seed=6)
+    out = []
+    for n, per_degree in ((256, 2), (257, 3)):
+        f = lambda degree: es.chebyshev_filter(x[:, :n], V, 25.0, -2.0, 70.0, degree=degree)
+        n1 = _launches(ctx, lambda: f(2))[1]
+        y, n2 = _launches(ctx, lambda: f(3))
+        assert n2 - n1 == per_degree
+        out.append(y[:, :256])
+    eps = 2.0 ** -53 if precision == "fp64" else 2.0 ** -24
+    assert np.abs(out[0] - out[1]).max() < 100 * eps * np.abs(out[1]).max()
+    ctx.close()
+
+
+@pytest.mark.parametrize("block", [128, 37])
+def test_column_blocks_of_a_host_solve_take_one_route(synth_psp8, block):
+    """8 atoms and 300 columns are above the line, each block of the host solve's pipelined copy below it:
+    the line is the whole block's, so the two solves agree bitwise."""
+    import ctypes
+    from lynx_b200 import solver
+    cl, pos, V = _cell("si8", (20, 18, 20))
+    ctx = solver.Context(cl)
+    ctx.set_nonlocal(P.nonlocal_tables(cl, pos, P.read_psp8(synth_psp8)))
+    n, lo, hi = 300, float(V.min()) - 1.0, ctx.max_eigval_half_lap + 8.0
+    x = C.random_orbitals(ctx.nd, n, seed=7)
+    want, e_want = solver.EigenSolver(ctx, "mixed").solve(x, V, 0.5 * (lo + hi), lo, hi, 5)
+    got, eig, lc = np.asfortranarray(x.copy()), np.zeros(n), ctypes.c_double()
+    ctx.set_option(_lib.OPT_HOST_COPY_BLOCK, block)
+    _lib.check(ctx.lib.lynx_eigensolver_solve_host(ctx.handle, _lib.dptr(got), _lib.dptr(eig),
+                                                   _lib.dptr(np.ascontiguousarray(V)), n, ctx.nd, 0.5 * (lo + hi), lo,
+                                                   hi, 5, _lib.PREC_MIXED, ctypes.byref(lc)))
+    assert np.array_equal(eig, e_want) and np.array_equal(got, want)
+    ctx.close()
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("shape,ncol", [((20, 21, 22), 7), ((24, 24, 24), 1), ((22, 24, 26), 17)])
 def test_direct_step_is_the_pipelined_one(synth_psp8, precision, shape, ncol):
