@@ -28,9 +28,9 @@ cudaError_t smem_cap(K* kern, size_t bytes) {
 
 // Programmatic dependent launch for the chains of short kernels of the filter: the next kernel's blocks
 // may be set up while this one still runs, and wait in pdl_wait() for all of its results.  Every kernel
-// launched this way calls pdl_wait() before it touches memory that an earlier kernel may read or write,
-// and in every thread, also where there is nothing to do: a wait covers the grid before it only, so a grid
-// that ends without waiting would let the next one start on results that are still being written.
+// launched this way calls pdl_wait() before it touches memory that an earlier kernel may read or write.
+// A wait covers the grid before it only, so every grid must hold a block that waits: one whose blocks all
+// leave early would let the next kernel start on results that are still being written.
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_wait() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -116,10 +116,7 @@ __global__ void __launch_bounds__(256)
     const S* chi = reinterpret_cast<const S*>(tab.chi);
     const int a = blockIdx.y;
     const int np = tab.atom_nproj[a];
-    if (np == 0) {
-        pdl_wait();  // the next kernel's wait covers this grid only
-        return;
-    }
+    if (np == 0) return;  // another atom has projectors (launch_atom_kernel), and its blocks wait
     const int poff = tab.atom_poff[a];
     const int i0 = tab.atom_img_ptr[a], i1 = tab.atom_img_ptr[a + 1];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;

@@ -80,6 +80,9 @@ namespace {
 template <typename T, bool APPLY>
 int launch_atom_kernel(const NLDev& nl, const T* x, long long ld, int ncol, T* alpha, int ncolp, double dV, T* out,
                        long long ldo, typename ScalarOf<T>::type scale, cudaStream_t st) {
+    // Blocks of an atom without projectors leave at once; a grid of such blocks alone would end before the
+    // kernel ahead of it, and the kernel after it waits for this grid only.
+    if (nl.max_np == 0) return LYNX_OK;
     auto go = [&](auto kern, int nc) {
         dim3 grid(((APPLY ? ncol : ncolp) + nc - 1) / nc, nl.n_atom);
         launch_pdl(kern, grid, 256, 0, st, x, ld, ncol, ncolp, make_view<T>(nl), alpha, dV, out, ldo, scale);
@@ -112,7 +115,7 @@ int launch_nl_gather(const NLDev& nl, const T* x, long long ld, int ncol, T* alp
 template <typename T>
 int launch_nl_apply(const NLDev& nl, const T* x, long long ld, T* out, long long ldo, int ncol, double dV,
                     typename ScalarOf<T>::type scale, cudaStream_t st) {
-    if (nl.n_atom == 0 || nl.max_np == 0 || ncol <= 0) return LYNX_OK;
+    if (nl.n_atom == 0 || ncol <= 0) return LYNX_OK;
     if (!nl.compact || nl.max_np > 32) {
         set_error("the one-kernel nonlocal apply needs disjoint projector spheres and at most 32 projectors");
         return LYNX_ERR_UNSUPPORTED;

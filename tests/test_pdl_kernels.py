@@ -1,5 +1,6 @@
-"""Kernels of programmatic dependent launches: every thread waits for the grid before it, whatever it has
-to do.  Read off the sources (no GPU): what a kernel does not wait for depends on timing."""
+"""Kernels of programmatic dependent launches: no grid ends before the grid ahead of it.  Either no thread
+leaves before its wait, or the launch is left out where every block would.  Read off the sources (no
+GPU): what a kernel does not wait for depends on timing."""
 import os
 import re
 
@@ -33,8 +34,21 @@ def test_the_kernels_are_found():
     assert {k[0] for k in KERNELS} >= {"direct_step_kernel", "nonorth_mixed_kernel", "nl_atom_kernel"}
 
 
+# kernels some of whose blocks leave early: where they are launched, and what is asked before
+GUARDED = {"nl_atom_kernel": ("nonlocal_launch.cu", "launch_atom_kernel", "if (nl.max_np == 0) return LYNX_OK;")}
+
+
 @pytest.mark.parametrize("name,params,body", KERNELS, ids=[k[0] for k in KERNELS])
-def test_no_return_before_the_wait(name, params, body):
-    waits = [m.start() for m in re.finditer(r"pdl_wait\(\);", body)]
-    for m in re.finditer(r"\breturn;", body):
-        assert waits[0] < m.start(), f"{name} leaves before pdl_wait()"
+def test_no_grid_leaves_before_the_wait(name, params, body):
+    wait = body.index("pdl_wait();")
+    early = [m.start() for m in re.finditer(r"\breturn;", body) if m.start() < wait]
+    if name not in GUARDED:
+        assert not early, f"{name} leaves before pdl_wait()"
+        return
+    assert len(early) == 1 and "if (np == 0) return;" in body[:wait]
+    path, launcher, guard = GUARDED[name]
+    with open(os.path.join(CSRC, path)) as fh:
+        src = fh.read()
+    assert src.count(name + "<") == src.count("go(" + name + "<")  # one launcher
+    text = src[src.index("int " + launcher + "("):]
+    assert -1 < text.find(guard) < text.index("launch_pdl(")
