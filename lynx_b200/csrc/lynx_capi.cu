@@ -1424,6 +1424,13 @@ int rayleigh_ritz_small(lynx_ctx* c, const T* Y, const T* HY, long long ldb, int
     return finish_rr(c, N, eig_host);
 }
 
+// Mixed precision above kSmallRRMax states: products of 23-bit digits on the tensor cores, or FP64 products of
+// the FP32 blocks where the caller wants them and for odd nx.  Those blocks had FP64 products before their
+// rows were padded for the pipelined stencil, and the digits would take bits from the result: over 49^3 to
+// 61^3 points and 145 to 179 states the density lies 8.4e-8 from its 64-bit value with digits, 3.9e-8 with
+// FP64 products (relative 2-norm; the Ritz values 4e-8 either way).
+bool use_tc_products(const lynx_ctx* c) { return c->nx % 2 == 0 && !c->no_tc_gram; }
+
 // ---------------------------------------------------------------------------
 // CheFSI pass.  T64 = FP64 storage type (double / double2), T32 = FP32 (float / float2).
 // ---------------------------------------------------------------------------
@@ -1468,14 +1475,14 @@ int solve_impl(lynx_ctx* c, T64* psi, double* eig, const double* veff, int N, in
             return LYNX_OK;
         }
         if constexpr (std::is_same<T32, float>::value) {
-            if (pipe_capable<float>(c) && !c->no_tc_gram) {
+            if (use_tc_products(c)) {
                 LYNX_TRY(rayleigh_ritz_mixed_real(c, Y, HY, ldb, nxp, reinterpret_cast<double*>(psi), ldp, N, eig));
                 LYNX_TRY(check_errflag(c));
                 if (lc_out) *lc_out = eig[N - 1] + 0.1;
                 return LYNX_OK;
             }
         } else {
-            if (pipe_capable<float>(c) && rot_supported(2 * N) && !c->no_tc_gram) {
+            if (use_tc_products(c) && rot_supported(2 * N)) {
                 LYNX_TRY(rayleigh_ritz_mixed_cplx(c, Y, HY, ldb, nxp, reinterpret_cast<double2*>(psi), ldp, N, eig));
                 LYNX_TRY(check_errflag(c));
                 if (lc_out) *lc_out = eig[N - 1] + 0.1;

@@ -1,6 +1,6 @@
-"""Odd nx in the pipelined stencil (padded rows, element-wise wrapped x neighbours) and in the
-tensor-core Rayleigh-Ritz step that its padded blocks allow, against the numpy oracle; rows that end
-one or two points past a thread block, with and without the fused nonlocal term."""
+"""Odd nx in the pipelined stencil (padded rows, element-wise wrapped x neighbours) against the numpy
+oracle, rows that end one or two points past a thread block, with and without the fused nonlocal term;
+and the mixed pass, whose products stay FP64 for odd nx."""
 import numpy as np
 import pytest
 
@@ -40,8 +40,8 @@ def test_filter(synth_psp8, shape, precision, tol, fuse):
 
 @pytest.mark.parametrize("n", [41, 130])
 def test_mixed_pass(synth_psp8, n):
-    """The tensor-core products of odd rows against FP64 library products of the same filtered block,
-    and the density accumulated in the rotation against the density of the orbitals."""
+    """The products of odd rows are FP64 products of the filtered block with and without the tensor-core
+    option, bitwise; orthonormal orbitals, and the density that comes with the pass is theirs."""
     import torch
     solver, ctx, V, _ = _system(synth_psp8, 1, (25, 26, 27))
     es = solver.EigenSolver(ctx, "mixed")
@@ -55,7 +55,21 @@ def test_mixed_pass(synth_psp8, n):
         w = solver.electron_density(ctx, psi, solver.occupations(eig, ef, 1000.0))
         assert float((rho - w).abs().max()) < 1e-12 * float(w.abs().max())
         s = (psi @ psi.T).cpu().numpy() * ctx.dV
-        assert np.abs(s - np.eye(n)).max() < 1e-5
-        out.append(eig)
-    assert np.abs(out[0] - out[1]).max() < 2e-7 * np.abs(out[1]).max()
+        assert np.abs(s - np.eye(n)).max() < 1e-12
+        out.append((eig, psi.cpu().numpy()))
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+    ctx.close()
+
+
+def test_mixed_kpt_pass(synth_psp8):
+    solver, ctx, V, _ = _system(synth_psp8, 1, (25, 24, 23))
+    ctx.set_kpoint(np.array([0.25, -0.125, 0.375]) * 2 * np.pi / ctx.cell.lengths)
+    es = solver.EigenSolver(ctx, "mixed")
+    lo, hi = float(V.min()) - 1.0, ctx.max_eigval_half_lap + 8.0
+    out = []
+    for tc in (1, 0):
+        ctx.set_option(_lib.OPT_TC_RAYLEIGH_RITZ, tc)
+        x = C.random_orbitals(ctx.nd, 45, seed=3, complex_=True)
+        out.append(es.solve_kpt(x, V, 0.5 * (lo + hi), lo, hi, 6))
+    assert np.array_equal(out[0][1], out[1][1]) and np.array_equal(out[0][0], out[1][0])
     ctx.close()
