@@ -1,4 +1,5 @@
 // Launchers for the deterministic nonlocal gather / scatter kernels.
+#include <algorithm>
 #include <type_traits>
 #include "kernels.h"
 #include "lynx_common.cuh"
@@ -76,6 +77,7 @@ int gather2_dispatch(const NLDev& nl, const T* x, long long ld, int ncol, T* alp
 }  // namespace
 
 namespace {
+constexpr int kMaxGridY = 65535;
 // One CTA per (atom, NC columns).  NC x NP sums per lane fit the registers.
 template <typename T, bool APPLY>
 int launch_atom_kernel(const NLDev& nl, const T* x, long long ld, int ncol, T* alpha, int ncolp, double dV, T* out,
@@ -84,8 +86,20 @@ int launch_atom_kernel(const NLDev& nl, const T* x, long long ld, int ncol, T* a
     // kernel ahead of it, and the kernel after it waits for this grid only.
     if (nl.max_np == 0) return LYNX_OK;
     auto go = [&](auto kern, int nc) {
-        dim3 grid(((APPLY ? ncol : ncolp) + nc - 1) / nc, nl.n_atom);
-        launch_pdl(kern, grid, 256, 0, st, x, ld, ncol, ncolp, make_view<T>(nl), alpha, dV, out, ldo, scale);
+        const unsigned groups = ((APPLY ? ncol : ncolp) + nc - 1) / nc;
+        NLView v = make_view<T>(nl);
+        if (nl.n_atom <= kMaxGridY) {
+            launch_pdl(kern, dim3(groups, nl.n_atom), 256, 0, st, x, ld, ncol, ncolp, v, alpha, dV, out, ldo, scale);
+            return;
+        }
+        // more atoms than a grid's y extent: one launch after the other (a part may hold empty blocks alone)
+        for (int a0 = 0; a0 < nl.n_atom; a0 += kMaxGridY) {
+            const dim3 grid(groups, std::min(kMaxGridY, nl.n_atom - a0));
+            kern<<<grid, 256, 0, st>>>(x, ld, ncol, ncolp, v, alpha, dV, out, ldo, scale);
+            v.atom_img_ptr += kMaxGridY;
+            v.atom_nproj += kMaxGridY;
+            v.atom_poff += kMaxGridY;
+        }
     };
     constexpr int NC = std::is_same<T, float>::value ? 4 : std::is_same<T, double>::value ? 2 : 1;
     constexpr int NC32 = NC >= 2 ? NC / 2 : 1;

@@ -56,6 +56,26 @@ def test_h_apply_of_small_blocks(synth_psp8, kind, shape, ncol, kpt, fd_order):
     ctx.close()
 
 
+def test_complex_projections_of_very_many_atoms():
+    """70000 one-point atoms, above the extent of a grid in y, every other of the later ones without a
+    projector: the nonlocal term is then a factor per grid point (1e-14: sums of about 8 terms)."""
+    from lynx_b200 import solver
+    cl, _, _ = _cell("si8", (20, 21, 22))
+    n, r = 70000, np.random.default_rng(5)
+    nproj = np.ones(n, np.int32)
+    nproj[65535::2] = 0
+    chi, gamma, gpos = r.normal(size=nproj.sum()), r.normal(size=nproj.sum()), r.integers(0, cl.nd, n)
+    tab = P.NonlocalTables(np.arange(n, dtype=np.int32), np.ones(n, np.int32), np.zeros((n, 3)), np.zeros((n, 3)),
+                           gpos.astype(np.int32), chi, nproj, gamma)
+    ctx = solver.Context(cl)
+    ctx.set_nonlocal(tab)
+    x = C.random_orbitals(ctx.nd, 2, seed=4, complex_=True)
+    got = solver.NonlocalProjector(ctx).apply(x, np.zeros_like(x), kpt=True)
+    f = np.bincount(gpos[nproj > 0], weights=chi * chi * gamma * cl.dV, minlength=cl.nd)
+    assert np.abs(got - f[:, None] * x).max() < 1e-14 * np.abs(f).max()
+    ctx.close()
+
+
 def _launches(ctx, f):
     ctx.lib.lynx_launch_count(1)
     out = f()
