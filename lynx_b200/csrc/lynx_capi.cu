@@ -2484,6 +2484,12 @@ int stress_impl(lynx_ctx* c, const T* psi, int nband, int ld, const double* occ,
     const long long l = ld > 0 ? ld : c->Nd;
     LYNX_CHECK_ARG(l >= c->Nd, "ld < Nd");
     LYNX_CHECK_ARG(!c->has_nl || img_pos, "image positions are required when projectors are set");
+    if (!c->orth) {
+        const double* u = c->uvec;
+        const double det = u[0] * (u[4] * u[8] - u[5] * u[7]) - u[1] * (u[3] * u[8] - u[5] * u[6]) +
+                           u[2] * (u[3] * u[7] - u[4] * u[6]);
+        LYNX_CHECK_ARG(std::fabs(det) > 1e-14, "singular lattice");
+    }
     LYNX_TRY(activate(c));
     const int na = c->has_nl ? c->nl.n_atom : 0;
     const ForceGeom g = force_geom(c);

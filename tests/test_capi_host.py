@@ -150,3 +150,20 @@ def test_spline_reproduces_cubics():
     xi = np.linspace(0.05, 2.95, 97)
     np.testing.assert_allclose(P.spline_eval(x, y, s, xi), 1.0 - 2.0 * xi + 0.5 * xi ** 2 - 0.3 * xi ** 3,
                                atol=1e-12)
+
+
+@pytest.mark.parametrize("entry", ["lynx_kinetic_nonlocal_stress", "lynx_kinetic_nonlocal_stress_kpt"])
+def test_stress_of_a_singular_lattice_is_refused(entry):
+    """Unit lattice vectors whose determinant is 1e-16, in a cell large enough to be taken by
+    lynx_create: the Cartesian gradients do not exist.  (Refused before any work on a device.)"""
+    lib = _lib.load()
+    h = ctypes.c_void_p()
+    lat = np.array([[1e4, 0, 0], [0, 1e4, 0], [1e4, 0, 1e-12]])
+    _lib.check(lib.lynx_create(ctypes.byref(h), 0, 16, 16, 16, 12, _lib.dptr(lat), 0, None))
+    try:
+        occ, psi, out = np.ones(1), np.zeros(2 * 16 ** 3), np.zeros(12)
+        rc = getattr(lib, entry)(h, ctypes.c_void_p(psi.ctypes.data), 1, 0, _lib.dptr(occ), 2.0, None,
+                                 _lib.dptr(out[:6]), _lib.dptr(out[6:]))
+        assert rc == _lib.LYNX_ERR_BAD_ARG and b"singular lattice" in lib.lynx_last_error()
+    finally:
+        lib.lynx_destroy(h)
