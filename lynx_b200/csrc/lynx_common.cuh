@@ -30,7 +30,9 @@ cudaError_t smem_cap(K* kern, size_t bytes) {
 // may be set up while this one still runs, and wait in pdl_wait() for all of its results.  Every kernel
 // launched this way calls pdl_wait() before it touches memory that an earlier kernel may read or write.
 // A wait covers the grid before it only, so every grid must hold a block that waits: one whose blocks all
-// leave early would let the next kernel start on results that are still being written.
+// leave early would let the next kernel start on results that are still being written.  Pointers to
+// earlier results are not `const __restrict__`: that reads through the path for data that is constant while
+// the kernel lives, and this kernel lives before its predecessor has written.
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_wait() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

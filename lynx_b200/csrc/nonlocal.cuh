@@ -107,8 +107,8 @@ constexpr int fold_slots() {  // values left per lane after R rounds
 constexpr int kAtomImgs = 32;
 template <typename T, int NP, int NC, bool APPLY>
 __global__ void __launch_bounds__(256)
-    nl_atom_kernel(const T* __restrict__ x, long long ld, int ncol, int ncolp, NLView tab, T* __restrict__ alpha,
-                   double dV, T* __restrict__ out, long long ldo, typename ScalarOf<T>::type scale) {
+    nl_atom_kernel(const T* x, long long ld, int ncol, int ncolp, NLView tab, T* alpha, double dV, T* out,
+                   long long ldo, typename ScalarOf<T>::type scale) {
     using S = typename ScalarOf<T>::type;
     constexpr int M = NP * NC;
     __shared__ T red[8][M];

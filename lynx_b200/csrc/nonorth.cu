@@ -70,8 +70,8 @@ __global__ void __launch_bounds__(256)
 
 template <typename T, int R>  // R: the half-width (unrolled: all 6 R loads in flight)
 __global__ void __launch_bounds__(128)
-    nonorth_mixed_kernel(const T* __restrict__ gy, const T* __restrict__ gz, long long ldg, T* __restrict__ out,
-                         long long ldout, typename ScalarOf<T>::type scale, const NOArgs<T> A) {
+    nonorth_mixed_kernel(const T* gy, const T* gz, long long ldg, T* out, long long ldout,
+                         typename ScalarOf<T>::type scale, const NOArgs<T> A) {
     pdl_wait();
     const int np = A.nx * A.ny * A.nz;
     const int t = blockIdx.x * 128 + threadIdx.x;

@@ -43,9 +43,8 @@ struct DirectArgs {
 
 template <typename T, int R, bool XOLD, bool GRAD>
 __global__ void __launch_bounds__(128)
-    direct_step_kernel(const T* __restrict__ x, const T* __restrict__ xold, T* __restrict__ out,
-                       const typename ScalarOf<T>::type* __restrict__ V, T* __restrict__ gy, T* __restrict__ gz,
-                       const DirectArgs<T> A) {
+    direct_step_kernel(const T* x, const T* xold, T* __restrict__ out, const typename ScalarOf<T>::type* V,
+                       T* __restrict__ gy, T* __restrict__ gz, const DirectArgs<T> A) {
     using S = typename ScalarOf<T>::type;
     pdl_wait();
     const int t = blockIdx.x * 128 + threadIdx.x;

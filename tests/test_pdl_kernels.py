@@ -1,6 +1,7 @@
 """Kernels of programmatic dependent launches: no grid ends before the grid ahead of it.  Either no thread
-leaves before its wait, or the launch is left out where every block would.  Read off the sources (no
-GPU): what a kernel does not wait for depends on timing."""
+leaves before its wait, or the launch is left out where every block would.  And what the grid ahead may
+write is not read as data that is constant for the kernel's life.  Read off the sources (no GPU): what
+a kernel does not wait for depends on timing."""
 import os
 import re
 
@@ -52,3 +53,8 @@ def test_no_grid_leaves_before_the_wait(name, params, body):
     assert src.count(name + "<") == src.count("go(" + name + "<")  # one launcher
     text = src[src.index("int " + launcher + "("):]
     assert -1 < text.find(guard) < text.index("launch_pdl(")
+
+
+@pytest.mark.parametrize("name,params,body", KERNELS, ids=[k[0] for k in KERNELS])
+def test_no_constant_pointers(name, params, body):
+    assert not re.search(r"\bconst\b[^,]*\*\s*__restrict__", params) and "__ldg(" not in body
