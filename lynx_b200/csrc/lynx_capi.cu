@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <array>
 #include <atomic>
+#include <climits>
 #include <cmath>
 #include <cstdarg>
 #include <cstdlib>
@@ -1743,6 +1744,10 @@ int lynx_create(lynx_ctx** out, int device, int nx, int ny, int nz, int fd_order
     LYNX_CHECK_ARG(out != nullptr && latvec != nullptr, "null pointer");
     *out = nullptr;
     LYNX_CHECK_ARG(nx > 0 && ny > 0 && nz > 0, "grid dimensions must be positive");
+    // Grid points are counted in 32 bits: by the thread of a block of up to 128 past the last point, and in
+    // rows rounded up to four elements.
+    LYNX_CHECK_ARG((nx + 3LL) / 4 * 4 * ny <= INT_MAX / nz && (nx + 3LL) / 4 * 4 * ny * nz <= INT_MAX - 128,
+                   "more grid points than 32-bit indices hold");
     LYNX_CHECK_ARG(fd_order >= 2 && fd_order % 2 == 0, "FD order must be even and >= 2");
     lynx_ctx* c = new lynx_ctx();
     c->device = device;

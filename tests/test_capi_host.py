@@ -167,3 +167,20 @@ def test_stress_of_a_singular_lattice_is_refused(entry):
         assert rc == _lib.LYNX_ERR_BAD_ARG and b"singular lattice" in lib.lynx_last_error()
     finally:
         lib.lynx_destroy(h)
+
+
+@pytest.mark.parametrize("shape,taken", [((1289, 1289, 1289), True), ((1290, 1290, 1290), False),
+                                         ((1291, 1291, 1291), False), ((509, 2048, 2048), False),
+                                         ((2147483520, 1, 1), False), ((2147483516, 1, 1), True),
+                                         ((65536, 65536, 65536), False)])
+def test_grids_beyond_32_bit_indices_are_refused(shape, taken):
+    """The count of padded points (rows rounded up to four) and a thread block past them stay below 2^31."""
+    lib = _lib.load()
+    h = ctypes.c_void_p()
+    lat = np.eye(3) * 100.0
+    rc = lib.lynx_create(ctypes.byref(h), 0, *shape, 12, _lib.dptr(lat), 1, None)
+    assert rc == (_lib.LYNX_OK if taken else _lib.LYNX_ERR_BAD_ARG)
+    if taken:
+        lib.lynx_destroy(h)
+    else:
+        assert not h.value and b"32-bit" in lib.lynx_last_error()
