@@ -35,9 +35,10 @@ template <typename T>
 int launch_nonorth_terms(const NonOrthGeom& g, int nxp, const T* x, long long ldx, T* gy, T* gz, long long ldg, T* out,
                          long long ldout, int ncol, double a, const T* phl, const T* phr, cudaStream_t st,
                          bool have_grads = false);
-// The Chebyshev step of small problems, one thread per point (stencil_direct.cu, FD order 12, any
-// row pitch and alignment).  ng (may be null): also write the first derivatives of x along y and z
+// The Chebyshev step of complex blocks and small real ones, one thread per point (stencil_direct.cu,
+// any half-width, row pitch and alignment).  ng (may be null): also write the first derivatives of x along y and z
 // to gy and gz (column stride ldg).
+constexpr int kDirectMaxNx = 512;  // longest rows of the direct step
 template <typename T, typename S>
 int launch_direct_step(const StencilGeom& g, int nxp, const T* x, long long ldx, const T* xold, long long ldo, T* out,
                        long long ldout, const S* V, int ncol, double a, double b, double d, const T* phl,

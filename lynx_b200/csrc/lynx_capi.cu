@@ -864,8 +864,8 @@ int stencil_time_add(lynx_ctx* c) {
 // The one-thread-per-point kernel (stencil_direct.cu) takes complex blocks, and real ones that are
 // small enough to be bound by latency (both sides measured: see that file).
 constexpr long long kDirectRealBytes = 1250000;
-template <typename T> bool direct_step_pays(long long nd, int ncol) {
-    return ScalarOf<T>::cplx || nd * ncol * (long long)sizeof(T) <= kDirectRealBytes;
+template <typename T> bool direct_step_pays(const lynx_ctx* c, int ncol) {
+    return c->nx <= kDirectMaxNx && c->Nd * (long long)ncol * (long long)sizeof(T) <= kDirectRealBytes;
 }
 
 // Columns of the block that a step's ncol columns belong to.
@@ -902,7 +902,7 @@ int cheb_step(lynx_ctx* c, int nxp, const T* x, long long ldx, const T* xold, lo
                       c->bc[1] == LYNX_BC_PERIODIC && c->bc[2] == LYNX_BC_PERIODIC;
     const long long ldw = ((long long)c->nl.n_pts + 3) & ~3LL;  // compact column stride
     const bool direct =
-        ScalarOf<T>::cplx || !pipe_ok || (!fuse && c->force_shape < 0 && direct_step_pays<T>(c->Nd, ncol));
+        ScalarOf<T>::cplx || !pipe_ok || (!fuse && c->force_shape < 0 && direct_step_pays<T>(c, ncol));
     const NLDev* nl = nullptr;
     if (c->has_nl) LYNX_TRY(nl_for(c, nxp, &nl));
     if (c->has_nl && !few) {

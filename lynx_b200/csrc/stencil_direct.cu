@@ -29,8 +29,6 @@
 namespace lynxb {
 namespace {
 
-constexpr int kDirectMaxNx = 512;
-
 template <typename T>
 struct DirectArgs {
     using S = typename ScalarOf<T>::type;

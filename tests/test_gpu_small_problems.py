@@ -82,6 +82,20 @@ def _launches(ctx, f):
     return out, ctx.lib.lynx_launch_count(0)
 
 
+@pytest.mark.parametrize("nx", [512, 514, 608])
+def test_small_blocks_of_long_rows(nx):
+    """Rows that the direct step does not take (above 512) run the pipelined kernel, small block or not."""
+    from lynx_b200 import solver
+    cl = C.Cell(np.diag([nx * 0.35, 5.0, 5.5]), (nx, 14, 16))
+    V = np.random.default_rng(2).normal(size=cl.nd)
+    x = C.random_orbitals(cl.nd, 1, seed=3)
+    ctx = solver.Context(cl)
+    y = solver.Hamiltonian(ctx, V).apply(x)
+    want = O.Operator(cl.latvec, cl.shape).apply(x, V)
+    assert np.abs(y - want).max() < 1e-12 * np.abs(want).max()
+    ctx.close()
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 def test_atom_kernel_up_to_2048_pairs(synth_psp8, precision):
     """8 atoms: 256 columns take the one-kernel apply (two launches a degree), 257 the staged gather, the
