@@ -180,7 +180,6 @@ int launch_cheb_pipe(const StencilGeom& g, int nxp, const T* x, long long ldx, c
         const int ty_bal = (g.ny + nb - 1) / nb;
         TYT = std::max(1, std::min(TYT, (ty_bal + RY - 1) / RY));
     }
-    const int nthr = ((P2 * TYT + 31) / 32) * 32 + 32;  // consumer warps + one producer warp
     PipeGeom G;
     G.nx = g.nx;
     G.ny = g.ny;
@@ -188,22 +187,12 @@ int launch_cheb_pipe(const StencilGeom& g, int nxp, const T* x, long long ldx, c
     G.nxp = nxp;
     G.GL = 0;
     G.SP = nxp;
-    G.TYT = TYT;
-    G.TY = TYT * RY;
     G.P2 = P2;
     G.plane = (long long)nxp * g.ny;
     G.ld_x = ldx;
     G.ld_old = ldo;
     G.ld_out = ldout;
-    const int nbands = (g.ny + G.TY - 1) / G.TY;
-    const long long base = (long long)nbands * ncol;
-    int nzch = (int)std::min<long long>((600 + base - 1) / base, std::max(1, g.nz / (4 * R)));
-    if (base * nzch < kFewCtas) nzch = (int)std::min<long long>((kFewCtas + base - 1) / base, g.nz / kMinChunk);
-    nzch = std::max(1, nzch);
-    G.zchunk = (g.nz + nzch - 1) / nzch;
-    nzch = (g.nz + G.zchunk - 1) / G.zchunk;
     const bool xo = (xold != nullptr) && d != 0.0;
-    const size_t own_b = (size_t)G.TY * nxp * sizeof(T);
     PipeNL<T> NL{};
     if (nlf) {
         NL.W = static_cast<const T*>(nlh->W);
@@ -212,28 +201,51 @@ int launch_cheb_pipe(const StencilGeom& g, int nxp, const T* x, long long ldx, c
         NL.mp = nlh->mp;
         NL.rowstart = nlh->rowstart;
         NL.xs_out = static_cast<T*>(nlh->xs_out);
-        // largest 16-byte-rounded W range of one band-plane for this band height
-        const int VWn = 16 / (int)sizeof(T);
-        const std::vector<int>& rs = *nlh->rowstart_host;
-        int wcap = 0;
-        for (int z = 0; z < g.nz; ++z)
-            for (int y0 = 0; y0 < g.ny; y0 += G.TY) {
-                const int tyv = std::min(G.TY, g.ny - y0);
-                const int ps = rs[(size_t)z * g.ny + y0], pe = rs[(size_t)z * g.ny + y0 + tyv];
-                wcap = std::max(wcap, ((pe + VWn - 1) & ~(VWn - 1)) - (ps & ~(VWn - 1)));
-            }
-        NL.wcap = wcap;
     }
-    const size_t stage = (size_t)pipe_stage_layout(G.TY, R, nxp, (int)sizeof(T), (int)sizeof(S), xo, nlf, NL.mp,
-                                                   NL.wcap).bytes;
-    // window ring (4 stages of the band's own rows) + as many tile stages (3..5) as fit
-    const size_t wring = 4 * ((own_b + 127) / 128) * 128 + (nlf ? (size_t)8 * G.zchunk : 0);  // + W range table
-    int ns = (int)std::min<size_t>(5, (227 * 1024 - 256 - wring) / stage);
-    const size_t smem = 256 + wring + (size_t)std::max(ns, 3) * stage;
-    if (smem > 227 * 1024) {
+    constexpr size_t kSmemMax = 227 * 1024;
+    int nbands = 0, nzch = 0, ns = 0;
+    // bands of tyt thread rows: z chunks, stages, and the shared memory they take
+    auto plan = [&](int tyt) -> size_t {
+        G.TYT = tyt;
+        G.TY = tyt * RY;
+        nbands = (g.ny + G.TY - 1) / G.TY;
+        const long long base = (long long)nbands * ncol;
+        nzch = (int)std::min<long long>((600 + base - 1) / base, std::max(1, g.nz / (4 * R)));
+        if (base * nzch < kFewCtas) nzch = (int)std::min<long long>((kFewCtas + base - 1) / base, g.nz / kMinChunk);
+        nzch = std::max(1, nzch);
+        G.zchunk = (g.nz + nzch - 1) / nzch;
+        nzch = (g.nz + G.zchunk - 1) / G.zchunk;
+        const size_t own_b = (size_t)G.TY * nxp * sizeof(T);
+        if (nlf) {
+            // largest 16-byte-rounded W range of one band-plane for this band height
+            const int VWn = 16 / (int)sizeof(T);
+            const std::vector<int>& rs = *nlh->rowstart_host;
+            int wcap = 0;
+            for (int z = 0; z < g.nz; ++z)
+                for (int y0 = 0; y0 < g.ny; y0 += G.TY) {
+                    const int tyv = std::min(G.TY, g.ny - y0);
+                    const int ps = rs[(size_t)z * g.ny + y0], pe = rs[(size_t)z * g.ny + y0 + tyv];
+                    wcap = std::max(wcap, ((pe + VWn - 1) & ~(VWn - 1)) - (ps & ~(VWn - 1)));
+                }
+            NL.wcap = wcap;
+        }
+        const size_t stage = (size_t)pipe_stage_layout(G.TY, R, nxp, (int)sizeof(T), (int)sizeof(S), xo, nlf, NL.mp,
+                                                       NL.wcap).bytes;
+        // window ring (4 stages of the band's own rows) + as many tile stages (3..5) as fit
+        const size_t wring = 4 * ((own_b + 127) / 128) * 128 + (nlf ? (size_t)8 * G.zchunk : 0);  // + W range table
+        ns = (int)std::min<size_t>(5, (kSmemMax - 256 - wring) / stage);
+        return 256 + wring + (size_t)std::max(ns, 3) * stage;
+    };
+    size_t smem = plan(TYT);
+    // Odd nx has one compiled shape (the caller tries the others where an even nx does not fit): with
+    // densely packed spheres the W ranges of a band can be too long for it, in FP32 from rows of about 120
+    // points on, and shorter bands fit.
+    while (odd && smem > kSmemMax && TYT > 1) smem = plan(--TYT);
+    if (smem > kSmemMax) {
         set_error("pipelined stencil stage of %zu bytes exceeds shared memory", smem);
         return LYNX_ERR_UNSUPPORTED;
     }
+    const int nthr = ((P2 * TYT + 31) / 32) * 32 + 32;  // consumer warps + one producer warp
     if (ncol > 65535 || nzch > 65535) {
         set_error("too many columns (%d) for one launch", ncol);
         return LYNX_ERR_UNSUPPORTED;

@@ -38,6 +38,30 @@ def test_filter(synth_psp8, shape, precision, tol, fuse):
     ctx.close()
 
 
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("shape", [(117, 48, 16), (237, 40, 12), (239, 20, 16)])
+def test_densely_packed_spheres(shape, precision):
+    """Every grid point in a sphere: a band's expanded values take as much shared memory as its rows, and
+    the bands are made shorter until the stages fit.  Bitwise the separate nonlocal term."""
+    from lynx_b200 import solver
+    cl = C.Cell(np.diag([n * 0.35 for n in shape]), shape)
+    nat, r = 36, np.random.default_rng(7)
+    gpos = np.arange(cl.nd, dtype=np.int32)
+    ndc = np.diff(np.linspace(0, cl.nd, nat + 1).astype(np.int32)).astype(np.int32)
+    tab = P.NonlocalTables(np.arange(nat, dtype=np.int32), ndc, np.zeros((nat, 3)), np.zeros((nat, 3)), gpos,
+                           r.normal(size=2 * cl.nd), np.full(nat, 2, np.int32), 1e-3 * r.normal(size=2 * nat))
+    ctx = solver.Context(cl)
+    ctx.set_nonlocal(tab)
+    V = r.normal(size=cl.nd)
+    x = C.random_orbitals(ctx.nd, 40, seed=3)
+    out = []
+    for fuse in (1, 0):
+        ctx.set_option(_lib.OPT_FUSE_NONLOCAL, fuse)
+        out.append(solver.EigenSolver(ctx, precision).chebyshev_filter(x, V, 25.0, -9.0, 75.0, degree=3))
+    assert np.array_equal(out[0], out[1])
+    ctx.close()
+
+
 @pytest.mark.parametrize("n", [41, 130])
 def test_mixed_pass(synth_psp8, n):
     """The products of odd rows are FP64 products of the filtered block with and without the tensor-core
