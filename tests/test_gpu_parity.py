@@ -33,6 +33,31 @@ def system(synth_psp8):
     return dict(cell=cl, pos=pos, V=V, R=R, ctx=ctx, solver=solver, torch=torch, synth_psp8=synth_psp8)
 
 
+@pytest.fixture(scope="module")
+def plain(synth_psp8):
+    """The same system for tests that need no reference."""
+    from lynx_b200 import solver
+    cl, pos, V = si8_small()
+    ctx = solver.Context(cl)
+    ctx.set_nonlocal(P.nonlocal_tables(cl, pos, P.read_psp8(synth_psp8)))
+    return dict(cell=cl, pos=pos, V=V, ctx=ctx, solver=solver, synth_psp8=synth_psp8)
+
+
+def _si64(shape):
+    """64 atoms (fewer than 32 take the one-kernel nonlocal apply instead of the fused term)."""
+    cl, pos = C.diamond_si(2, shape, displace=0.02, seed=6)
+    return cl, pos, C.synthetic_veff_separable(cl, pos, noise=1e-3, seed=6)
+
+
+def _launches_per_degree(ctx, es, X, V, bounds, prec):
+    n = []
+    for degree in (2, 3):
+        ctx.lib.lynx_launch_count(1)
+        es.chebyshev_filter(X, V, *bounds, degree, precision=prec)
+        n.append(ctx.lib.lynx_launch_count(0))
+    return n[1] - n[0]
+
+
 def test_grid_matches_reference(system):
     R, ctx = system["R"], system["ctx"]
     assert ctx.nd == R.nd
@@ -245,25 +270,30 @@ def test_mixed_pass_tensor_core_gram(system, nstates):
     assert subspace_distance(out["mixed"][0], out["fp64"][0]) < 1e-3
 
 
-def test_fused_nonlocal_and_shapes_bitwise(system):
+@pytest.mark.parametrize("shape", [(48, 50, 52), (50, 49, 51), (96, 48, 50)])
+def test_fused_nonlocal_and_shapes_bitwise(synth_psp8, shape):
     """The fused nonlocal term (stencil kernel adds a * chi alpha), with the projections read from
     the full grid or from the compact sphere-point copy the previous step wrote, and every launch
     shape give bitwise the results of the separate-scatter default-shape path (same operations,
-    same order)."""
-    from lynx_b200 import _lib
-    s = system
-    lo, hi, lc = _bounds(s)
-    X = C.random_orbitals(s["ctx"].nd, 20, seed=91)
+    same order).  Even, ragged and wide grids; z extents that recycle every ring stage of the fused
+    stencil several times, each stage carrying a different W range."""
+    from lynx_b200 import _lib, solver
+    cl, pos, V = _si64(shape)
+    tab = P.nonlocal_tables(cl, pos, P.read_psp8(synth_psp8))
+    X = C.random_orbitals(cl.nd, 7, seed=91)
+    bounds = (25.0, -2.0, 75.0)
     out = {}
     for fuse, tune, compact in ((0, 0, 0), (0, 1, 0), (1, 0, 0), (1, 1, 0), (1, 1, 1)):
-        ctx = s["solver"].Context(s["cell"])
-        ctx.set_nonlocal(P.nonlocal_tables(s["cell"], s["pos"], P.read_psp8(s["synth_psp8"])))
-        _lib.check(ctx.lib.lynx_set_option(ctx.handle, _lib.OPT_FUSE_NONLOCAL, fuse))
-        _lib.check(ctx.lib.lynx_set_option(ctx.handle, _lib.OPT_AUTOTUNE, tune))
-        _lib.check(ctx.lib.lynx_set_option(ctx.handle, _lib.OPT_COMPACT_GATHER, compact))
-        es = s["solver"].EigenSolver(ctx)
+        ctx = solver.Context(cl)
+        ctx.set_nonlocal(tab)
+        ctx.set_option(_lib.OPT_FUSE_NONLOCAL, fuse)
+        ctx.set_option(_lib.OPT_AUTOTUNE, tune)
+        ctx.set_option(_lib.OPT_COMPACT_GATHER, compact)
+        es = solver.EigenSolver(ctx)
         for prec in ("fp64", "mixed"):
-            out[(fuse, tune, compact, prec)] = es.chebyshev_filter(X, s["V"], lc, lo, hi, 6, precision=prec)
+            out[(fuse, tune, compact, prec)] = es.chebyshev_filter(X, V, *bounds, 6, precision=prec)
+            # gather, expansion and fused stencil, or gather, stencil and scatter; not the atom kernel
+            assert _launches_per_degree(ctx, es, X, V, bounds, prec) == 3
         ctx.close()
     for prec in ("fp64", "mixed"):
         ref_ = out[(0, 0, 0, prec)]
@@ -271,38 +301,15 @@ def test_fused_nonlocal_and_shapes_bitwise(system):
             assert np.array_equal(out[key + (prec,)], ref_), (key, prec)
 
 
-def test_fused_nonlocal_wide_rows_bitwise(synth_psp8):
-    """A wider grid (36 x 20 x 40) whose z extent recycles every ring stage of the fused stencil
-    several times, each stage carrying a different W range: the fused term and its compact copy
-    give bitwise the separate-scatter results in both precisions."""
-    from lynx_b200 import _lib, solver
-    cl, pos, V = si8_small(grid=(36, 20, 40), seed=5)
-    X = C.random_orbitals(int(np.prod(cl.shape)), 12, seed=93)
-    out = {}
-    for fuse, compact in ((0, 0), (1, 0), (1, 1)):
-        ctx = solver.Context(cl)
-        ctx.set_nonlocal(P.nonlocal_tables(cl, pos, P.read_psp8(synth_psp8)))
-        _lib.check(ctx.lib.lynx_set_option(ctx.handle, _lib.OPT_FUSE_NONLOCAL, fuse))
-        _lib.check(ctx.lib.lynx_set_option(ctx.handle, _lib.OPT_COMPACT_GATHER, compact))
-        es = solver.EigenSolver(ctx)
-        lo, hi = es.lanczos_bounds(V)
-        for prec in ("fp64", "mixed"):
-            out[(fuse, compact, prec)] = es.chebyshev_filter(X, V, 0.5 * (lo + hi), lo, hi, 5, precision=prec)
-        ctx.close()
-    for prec in ("fp64", "mixed"):
-        for key in ((1, 0), (1, 1)):
-            assert np.array_equal(out[key + (prec,)], out[(0, 0, prec)]), (key, prec)
-
-
 @pytest.mark.parametrize("block", [0, 64, 37])
-def test_host_solve_pipelined_matches_device(system, block):
+def test_host_solve_pipelined_matches_device(plain, block):
     """lynx_eigensolver_solve_host copies psi in column blocks on a second stream and filters
     each block as it lands (mixed precision, >= 256 states; default blocks of 128 columns, and
     LYNX_OPT_HOST_COPY_BLOCK 64 and 37): bitwise the device-pointer pass."""
     import ctypes
     from lynx_b200 import _lib
-    s = system
-    lo, hi, lc = _bounds(s)
+    s = plain
+    lo, hi, lc = -2.0, 75.0, 25.0
     N = 300
     psi0 = C.random_orbitals(s["ctx"].nd, N, seed=201)
     hp = np.asfortranarray(psi0.copy())
@@ -321,22 +328,26 @@ def test_host_solve_pipelined_matches_device(system, block):
     assert np.array_equal(hp, np.asarray(psi_d))
 
 
-def test_every_stencil_shape_bitwise(system):
+@pytest.mark.parametrize("shape", [(48, 50, 52), (52, 49, 50)])
+@pytest.mark.parametrize("fuse", [1, 0])
+def test_every_stencil_shape_bitwise(synth_psp8, shape, fuse):
     """Every compiled launch shape of the pipelined stencil and both band splits
-    (LYNX_OPT_STENCIL_SHAPE k = 1..8), with the fused nonlocal term: bitwise the default shape's
-    filter, both precisions."""
-    from lynx_b200 import _lib
-    s = system
-    lo, hi, lc = _bounds(s)
-    X = C.random_orbitals(s["ctx"].nd, 10, seed=95)
-    ctx = s["solver"].Context(s["cell"])
-    ctx.set_nonlocal(P.nonlocal_tables(s["cell"], s["pos"], P.read_psp8(s["synth_psp8"])))
-    es = s["solver"].EigenSolver(ctx)
+    (LYNX_OPT_STENCIL_SHAPE k = 1..8), with the fused nonlocal term and without: bitwise the default
+    shape's filter, both precisions."""
+    from lynx_b200 import _lib, solver
+    cl, pos, V = _si64(shape)
+    X = C.random_orbitals(cl.nd, 5, seed=95)
+    ctx = solver.Context(cl)
+    ctx.set_nonlocal(P.nonlocal_tables(cl, pos, P.read_psp8(synth_psp8)))
+    ctx.set_option(_lib.OPT_FUSE_NONLOCAL, fuse)
+    ctx.set_option(_lib.OPT_AUTOTUNE, 0)
+    es = solver.EigenSolver(ctx)
     out = {}
     for k in range(0, 9):
-        _lib.check(ctx.lib.lynx_set_option(ctx.handle, _lib.OPT_STENCIL_SHAPE, k))
+        ctx.set_option(_lib.OPT_STENCIL_SHAPE, k)
         for prec in ("fp64", "mixed"):
-            out[(k, prec)] = es.chebyshev_filter(X, s["V"], lc, lo, hi, 4, precision=prec)
+            out[(k, prec)] = es.chebyshev_filter(X, V, 25.0, -2.0, 75.0, 4, precision=prec)
+    assert _launches_per_degree(ctx, es, X, V, (25.0, -2.0, 75.0), "mixed") == 3
     ctx.close()
     for prec in ("fp64", "mixed"):
         for k in range(1, 9):

@@ -82,6 +82,36 @@ def _launches(ctx, f):
     return out, ctx.lib.lynx_launch_count(0)
 
 
+@pytest.mark.parametrize("ncol", [3, 40])  # below and above 1.25 MB in both precisions
+@pytest.mark.parametrize("kind", ["dirichlet", "dirichlet-odd", "fcc"])
+def test_both_stencils_of_phased_and_skewed_cells(synth_psp8, kind, ncol):
+    """Dirichlet directions (zero ghosts) and real blocks of a non-orthogonal cell, with the direct step and
+    with the pipelined kernel (and the separate derivative kernels of the skewed cell): H psi and both
+    filters against the oracle.  Tolerances as for the periodic cells: 1e-12, 1e-10, 2e-5."""
+    from lynx_b200 import solver
+    if kind == "fcc":
+        cl, pos, V = _cell("fcc", (20, 20, 20))
+        tab = P.nonlocal_tables(cl, pos, P.read_psp8(synth_psp8))
+        H = _oracle(cl, tab)
+    else:
+        shape = (20, 22, 24) if kind == "dirichlet" else (21, 22, 20)
+        cl = C.Cell(C.diamond_si(1, 20)[0].latvec, shape, True, (1, 0, 1), 12)
+        V, tab = np.random.default_rng(4).normal(size=cl.nd), None
+        H = O.Operator(cl.latvec, cl.shape, order=12, orthogonal=True, bc=cl.bc)
+    ctx = solver.Context(cl)
+    ctx.set_nonlocal(tab)
+    x = C.random_orbitals(ctx.nd, ncol, seed=91)
+    y, want = solver.Hamiltonian(ctx, V).apply(x, shift=0.3), H.apply(x, V, 0.3)
+    assert np.abs(y - want).max() < 1e-12 * np.abs(want).max()
+    bounds = (25.0, -2.0, ctx.max_eigval_half_lap + 4.0)
+    want = O.chebyshev_filter(H, x, V, *bounds, 3)
+    es = solver.EigenSolver(ctx)
+    for prec, tol in (("fp64", 1e-10), ("mixed", 2e-5)):
+        y = es.chebyshev_filter(x, V, *bounds, 3, precision=prec)
+        assert np.abs(y - want).max() < tol * np.abs(want).max()
+    ctx.close()
+
+
 @pytest.mark.parametrize("nx", [512, 514, 608])
 def test_small_blocks_of_long_rows(nx):
     """Rows that the direct step does not take (above 512) run the pipelined kernel, small block or not."""
@@ -142,10 +172,10 @@ def test_column_blocks_of_a_host_solve_take_one_route(synth_psp8, block):
 
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
-@pytest.mark.parametrize("shape,ncol", [((20, 21, 22), 7), ((24, 24, 24), 1), ((22, 24, 26), 17)])
+@pytest.mark.parametrize("shape,ncol", [((20, 21, 22), 7), ((24, 24, 24), 1), ((22, 24, 26), 11)])
 def test_direct_step_is_the_pipelined_one(synth_psp8, precision, shape, ncol):
     """The same sums in the same order: bitwise the pipelined kernel's filter (forced by the launch
-    shape option)."""
+    shape option).  All blocks below 1.25 MB in FP64, where the direct step is the default."""
     from lynx_b200 import solver
     cl, pos, V = _cell("si8", shape)
     ctx = solver.Context(cl)
