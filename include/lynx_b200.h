@@ -13,8 +13,8 @@
  *   - Operator entry points take DEVICE pointers and run on the context's
  *     stream (lynx_set_stream).  The *_host entry points take host pointers.
  *     A call's work is complete when it returns; only lynx_nonlocal_apply,
- *     _kpt and _noalloc, lynx_pair_density and lynx_randomize_orbitals return
- *     with work in flight on the stream.
+ *     _kpt and _noalloc, lynx_pair_density and lynx_randomize_orbitals, _all
+ *     may return with work in flight on the stream.
  *   - Every call returns LYNX_OK or an error status; lynx_last_error() gives
  *     the message of the last failing call on the calling thread.  Nothing
  *     calls exit(): a CUDA or solver failure is reported, not fatal.
@@ -53,7 +53,8 @@ enum {
 /* Arithmetic of the CheFSI pass. */
 enum {
     LYNX_PREC_FP64 = 0,  /* plain FP64 everywhere */
-    LYNX_PREC_MIXED = 1  /* FP32 filter + exact int8-slice tensor-core Rayleigh-Ritz products, FP64 subspace algebra */
+    LYNX_PREC_MIXED = 1  /* FP32 filter, FP64 subspace algebra; Rayleigh-Ritz products of the FP32 blocks: exact
+                          * int8 slices on the tensor cores, or FP64 (LYNX_OPT_TC_RAYLEIGH_RITZ says when) */
 };
 
 enum { LYNX_BC_PERIODIC = 0, LYNX_BC_DIRICHLET = 1 };
@@ -361,16 +362,21 @@ LYNX_API int lynx_nonlocal_apply_noalloc(lynx_ctx* ctx, const double* psi, doubl
  *                            the default shape.
  *   LYNX_OPT_FUSE_NONLOCAL:  1 (default) adds the nonlocal term inside the stencil kernel when
  *                            the projector spheres are disjoint (real data, periodic orthogonal
- *                            cell, FD order 12), from a compact per-point expansion; 0 always
- *                            uses the separate gather and scatter kernels.
+ *                            cell, FD order 12), from a compact per-point expansion; 0 uses
+ *                            the separate gather and scatter kernels.  Without effect on fewer
+ *                            than 32 atoms with at most 2048 (atom, column) pairs, whose term is
+ *                            one kernel of its own.
  *   LYNX_OPT_TC_RAYLEIGH_RITZ: 1 (default) runs the mixed-precision pass's Gram products and
- *                            rotation on the tensor cores (exact int8 slices, as accurate as
- *                            FP64 products of the FP32 blocks to about 1e-8); 0 runs them as FP64
+ *                            rotation of more than 40 states and even nx on the tensor cores
+ *                            (exact int8 slices, as accurate as FP64 products of the FP32 blocks
+ *                            to about 1e-8); up to 40 states they are FP64 products in kernels of
+ *                            their own, for odd nx FP64 library products.  0 runs them all as FP64
  *                            library products on FP64 copies of the FP32 blocks (slower).
  *   LYNX_OPT_COMPACT_GATHER: with the fused nonlocal term, 1 makes every filter step also write
  *                            its output at the sphere points as a compact block, and the next
  *                            step's projections read that block instead of the full grid; 0
- *                            (default) reads the full grid.  Same results, bitwise.
+ *                            (default) reads the full grid.  Same results, bitwise.  Without
+ *                            effect where LYNX_OPT_FUSE_NONLOCAL has none.
  *   LYNX_OPT_POISSON_DIRECT: 1 (default) makes lynx_effective_potential solve the Poisson equation
  *                            of a periodic cell exactly by FFT (the discrete equation the AAR
  *                            iteration converges to, to rounding); 0 uses the AAR iteration.

@@ -78,7 +78,9 @@ int gather2_dispatch(const NLDev& nl, const T* x, long long ld, int ncol, T* alp
 
 namespace {
 constexpr int kMaxGridY = 65535;
-// One CTA per (atom, NC columns).  NC x NP sums per lane fit the registers.
+// One CTA per (atom, NC columns): NC x NP sums per lane fit the registers, so complex data take one column.
+// A degree at a k-point, FP32 / FP64, against the staged complex gather and kernels before: Si8 30^3, 64
+// columns 66 / 179 us (288 / 348), Si64 60^3, 160 columns 1.36 / 3.69 ms (2.76 / 6.23).
 template <typename T, bool APPLY>
 int launch_atom_kernel(const NLDev& nl, const T* x, long long ld, int ncol, T* alpha, int ncolp, double dV, T* out,
                        long long ldo, typename ScalarOf<T>::type scale, cudaStream_t st) {

@@ -9,6 +9,11 @@
 // straight from the (padded) block into the caller's layout.  FP32 blocks are multiplied in FP64, so
 // the products are those of the library path.
 //
+// The line at 40 states is what the register and task layout below holds.  Us a pass beyond its filter, 40
+// states here against 41 by library (mixed: tensor-core) products, FP64 / mixed: 30^3 517 / 513 against
+// 867 / 1022, 60^3 902 / 824 against 1136 / 1339, 90^3 1897 / 1784 against 1768 / 1878; at a k-point 20^3 605 / 593
+// against 1241 / 1035, 60^3 2151 / 1429 against 9681 / 1853.
+//
 // Subspace eigenproblem: cyclic Jacobi rotations (Golub and Van Loan, Matrix Computations, sec. 8.5),
 // N/2 disjoint pairs at a time (round-robin order); all 2 x 2 blocks of a round are updated at once,
 // so a round is two barriers.  Converged when no off-diagonal entry exceeds 2^-54 of the norm.

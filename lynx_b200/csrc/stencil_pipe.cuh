@@ -1,9 +1,9 @@
-// Pipelined fused Chebyshev-filter step for sm_100a (the filter's hot kernel):
+// Pipelined fused Chebyshev-filter step for sm_100a (the filter's hot kernel on real blocks; complex
+// ones run stencil_direct.cu):
 //   out = a * (-0.5 * Lap x + Veff .* x) + b * x + d * xold
 // (src/solvers/EigenSolver.cpp:586-607 recurrence, src/operators/Hamiltonian.cpp:127-174
-// stencil, src/parallel/HaloExchange.cpp:34-189 ghost rules: periodic wrap, Bloch phase
-// e^{-+ik_dL_d} on left/right ghosts, zero for Dirichlet), with the ghosts produced in
-// the kernel: no padded copy of x is ever written to HBM.
+// stencil, src/parallel/HaloExchange.cpp:34-189 ghost rules: periodic wrap, zero for Dirichlet), with
+// the ghosts produced in the kernel: no padded copy of x is ever written to HBM.
 //
 // Data layout: blocks of ncol columns, each column a z-major stack of planes of ny rows,
 // rows padded to nxp >= nx elements (nxp * sizeof(T) a multiple of 16 bytes, pad
@@ -19,10 +19,8 @@
 //       by vector global loads issued two planes ahead.
 // The shared-memory ring holds P+1 stages, so the copies for plane z+P are in flight
 // while plane z is computed: memory-level parallelism comes from the async copies, not
-// from resident warps.  x-ghost columns of a staged plane are filled by the threads
-// (periodic or Bloch) after its copies land.  Each thread computes an RX x RY block of
-// points (RX adjacent x, RY adjacent y) so the x/y neighbour reads are vector
-// shared-memory loads reused across the block.
+// from resident warps.  Each thread computes an RX x RY block of points (RX adjacent x, RY adjacent
+// y) so the x/y neighbour reads are vector shared-memory loads reused across the block.
 //
 // HBM traffic per update: x, xold and out once each (3 words).  Halo rows and Veff are
 // re-read from L2.
@@ -186,8 +184,8 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // xold and Veff rows; and, in a separate DW-stage ring, the rows of the plane entering the
 // z-window).  The other warps are consumers: each thread computes RX adjacent x points on
 // RY adjacent rows.  Staged rows carry no ghost columns: a consumer reads its x neighbours
-// through column offsets wrapped once at start-up, and PHASED instantiations (Bloch phases,
-// Dirichlet zeros) multiply wrapped neighbours in registers.  Per stage two mbarriers:
+// through column offsets wrapped once at start-up, and PHASED instantiations (Dirichlet zeros)
+// multiply wrapped neighbours in registers.  Per stage two mbarriers:
 // full (copies landed, tx-counted) and empty (every consumer warp done reading).
 template <typename T, int R, int RX, int RY, bool XOLD, int NS, bool PHASED, int MAXT, bool NLF, bool ODD>
 __global__ void __launch_bounds__(MAXT, 1)

@@ -29,7 +29,10 @@ template <typename T> struct NumShapes { static constexpr int value = 1; };
 template <> struct NumShapes<float> { static constexpr int value = 4; };
 template <> struct NumShapes<double> { static constexpr int value = 4; };
 constexpr int kTunedR = 6;  // FD order 12
-// Odd nx (kTunedR, periodic cells): one shape per type, the one the autotuner keeps most often.
+// Odd nx (kTunedR, periodic cells): one compiled shape per type.  Us a degree with the fused term, the kept
+// shape first, then the others in order.  FP32 (1; 0, 2, 3): 51x57x63, 97 columns, 211; 206, 182, 201;
+// 61x60x59, 160 columns, 340; 340, 321, 328; 121x60x60, 60 columns, 236; 238, 243, 253.  FP64 (2; 0, 1, 3): 260;
+// 291, 294, 296, 501; 541, 507, 497 and 389; 367, 395, 374.
 template <typename T> struct OddShape;
 template <> struct OddShape<float> { static constexpr int value = 1; };
 template <> struct OddShape<double> { static constexpr int value = 2; };
@@ -70,8 +73,8 @@ void launch_pipe_ph(int ns, dim3 grid, int nthr, size_t smem, cudaStream_t st, c
     kern<<<grid, nthr, smem, st>>>(x, xo, out, V, G, C, NL, err);
 }
 
-// Real data with periodic boundaries needs no phase on wrapped neighbours; complex data and
-// Dirichlet boundaries use the PHASED instantiation (default shape only).
+// Periodic boundaries need no factor on wrapped neighbours; Dirichlet boundaries use the PHASED
+// instantiation (default shape only).
 template <typename T, int R, bool XOLD>
 void launch_pipe(int si, int ns, bool phased, bool nlf, bool odd, dim3 grid, int nthr, size_t smem, cudaStream_t st, const T* x,
                  const T* xo, T* out, const typename ScalarOf<T>::type* V, const PipeGeom& G, const PipeCoef<T>& C,
